@@ -265,3 +265,34 @@ def test_ps2_is_unsupported(gpu):
     with pytest.raises(EmsesError) as e:
         g.grdcrt(2)
     assert e.value.code == ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("ppc", [(1, 3), (4, 31), (33, 5), (64, 2)])
+@pytest.mark.parametrize("order", ["sorted", "shuffled"])
+def test_deposit_groups(gpu, ppc, order):
+    """psolve1's current and charge's arrays with cells shared by few, some
+    and all lanes of a warp, warps that end in the middle of a cell, and a
+    buffer in no order: the sums differ from the oracle's by their order
+    only (at most some thousand FP64 terms a node: TOL)."""
+    c = case(n=(5, 4, 3), ppc=ppc, vth_scale=3.0)
+    cfg, eb, p, tp = build(c)
+    if order == "shuffled":
+        rng = np.random.default_rng(3)
+        p = np.concatenate([rng.permutation(p[:tp[0]]), rng.permutation(p[tp[0]:])])
+    g = Emses(cfg)
+    g.upload_particles(p, tp)
+    g.upload_field("eb", eb)
+    o = O.Oracle(cfg, p, tp, eb)
+    g.grdcrt(1)
+    o.grdcrt()
+    for name in ("aj", "ajdg"):
+        g.zero_field(name)
+    g.psolve1(1, 2, 1, None)
+    o.psolve1(2, 1)
+    pg, _ = g.download_particles()
+    assert same_particles(pg, o.pbuf)
+    g.charge(1, 2)
+    o.charge(2)
+    for name in ("aj", "ajdg", "rho", "rhodg"):
+        assert rel_l2(g.download_field(name), o.f[name]) < TOL, name
+    g.close()
