@@ -9,9 +9,13 @@
 //      first output slot.
 //   3. k_radix_scatter: every warp ranks its 512 keys item by item with
 //      __match_any_sync (stable within the warp), warps are offset by an
-//      exclusive scan of their per-digit counts, and each key goes to
-//      hist[digit, block] + warp offset + rank.  Ties keep input order, so
-//      the pass (and the sort) is stable.
+//      exclusive scan of their per-digit counts, the tile is put in digit
+//      order in shared memory, and each pair goes to hist[digit, block] + its
+//      place among the block's pairs of that digit.  Ties keep input order,
+//      so the pass (and the sort) is stable.  The reordering makes the
+//      writes runs of a digit's pairs (16 of them on the mean) instead of
+//      single words: 0.117 ms a pass against 0.208 for 16.8 M pairs (a pass
+//      moves 268 MB).
 #include <algorithm>
 
 #include "common.cuh"
@@ -93,25 +97,28 @@ __global__ void __launch_bounds__(SORT_THREADS) k_radix_hist(const uint32_t* __r
   hist[(int64_t)threadIdx.x * nblocks + blockIdx.x] = cnt[threadIdx.x];
 }
 
-__global__ void __launch_bounds__(SORT_THREADS) k_radix_scatter(const uint32_t* __restrict__ keys,
+__global__ void __launch_bounds__(SORT_THREADS, 4) k_radix_scatter(const uint32_t* __restrict__ keys,
                                                                 const uint32_t* __restrict__ vals, int64_t n,
                                                                 int shift, const uint32_t* __restrict__ offs,
                                                                 int nblocks, uint32_t* __restrict__ keys_out,
                                                                 uint32_t* __restrict__ vals_out) {
   __shared__ uint32_t wcnt[SORT_WARPS][RADIX];
+  __shared__ uint32_t first[RADIX];   // first place of a digit in the block's order
+  __shared__ uint32_t shift_to[RADIX];  // output slot of a digit's first pair, less first
+  __shared__ uint32_t warp_sum[SORT_WARPS];
+  __shared__ uint32_t sk[SORT_TILE], sv[SORT_TILE];
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < SORT_WARPS * RADIX; i += SORT_THREADS) (&wcnt[0][0])[i] = 0;
   __syncthreads();
   // warp w owns [base + w*512, base + (w+1)*512), item-major then lane
   int64_t wbase = (int64_t)blockIdx.x * SORT_TILE + (int64_t)warp * (SORT_ITEMS * 32);
-  uint32_t k[SORT_ITEMS], v[SORT_ITEMS], rank[SORT_ITEMS];
+  uint32_t k[SORT_ITEMS], rank[SORT_ITEMS];
   unsigned lt = (1u << lane) - 1u;
 #pragma unroll
   for (int it = 0; it < SORT_ITEMS; it++) {
     int64_t idx = wbase + it * 32 + lane;
     bool ok = idx < n;
     k[it] = ok ? keys[idx] : 0u;
-    v[it] = ok ? vals[idx] : 0u;
     uint32_t d = (k[it] >> shift) & (RADIX - 1);
     uint32_t tag = ok ? d : (0x100u | (uint32_t)lane);
     unsigned peers = __match_any_sync(0xffffffffu, tag);
@@ -126,25 +133,48 @@ __global__ void __launch_bounds__(SORT_THREADS) k_radix_scatter(const uint32_t* 
     __syncwarp();
   }
   __syncthreads();
-  // exclusive scan over warps, per digit (thread t owns digit t)
-  {
-    uint32_t run = 0;
+  // exclusive scan over warps, per digit, and over the digits (thread t owns
+  // digit t): the block's own order
+  uint32_t run = 0;
 #pragma unroll
-    for (int w = 0; w < SORT_WARPS; w++) {
-      uint32_t c = wcnt[w][threadIdx.x];
-      wcnt[w][threadIdx.x] = run;
-      run += c;
-    }
+  for (int w = 0; w < SORT_WARPS; w++) {
+    uint32_t c = wcnt[w][threadIdx.x];
+    wcnt[w][threadIdx.x] = run;
+    run += c;
   }
+  uint32_t incl = run;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
   __syncthreads();
+  uint32_t before = 0;
+#pragma unroll
+  for (int w = 0; w < SORT_WARPS; w++) before += w < warp ? warp_sum[w] : 0u;
+  first[threadIdx.x] = before + incl - run;
+  shift_to[threadIdx.x] = offs[(int64_t)threadIdx.x * nblocks + blockIdx.x] - first[threadIdx.x];
+  __syncthreads();
+  // the pairs in that order in shared memory, then out: a digit's pairs go to
+  // consecutive slots, so neighbouring threads write neighbouring words
 #pragma unroll
   for (int it = 0; it < SORT_ITEMS; it++) {
-    int64_t idx = wbase + it * 32 + lane;
+    const int64_t idx = wbase + it * 32 + lane;
     if (idx >= n) continue;
-    uint32_t d = (k[it] >> shift) & (RADIX - 1);
-    uint32_t pos = offs[(int64_t)d * nblocks + blockIdx.x] + wcnt[warp][d] + rank[it];
-    keys_out[pos] = k[it];
-    vals_out[pos] = v[it];
+    const uint32_t d = (k[it] >> shift) & (RADIX - 1);
+    const uint32_t at = first[d] + wcnt[warp][d] + rank[it];
+    sk[at] = k[it];
+    sv[at] = vals[idx];
+  }
+  __syncthreads();
+  const int here = (int)min((int64_t)SORT_TILE, n - (int64_t)blockIdx.x * SORT_TILE);
+#pragma unroll 4
+  for (int at = threadIdx.x; at < here; at += SORT_THREADS) {
+    const uint32_t key = sk[at];
+    const uint32_t pos = shift_to[(key >> shift) & (RADIX - 1)] + at;
+    keys_out[pos] = key;
+    vals_out[pos] = sv[at];
   }
 }
 
