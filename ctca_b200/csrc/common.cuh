@@ -207,6 +207,8 @@ struct emsesg_ctx {
   EsState es;
   double* node64 = nullptr;            // drop-in node field: 8 doubles / node
   double* tj = nullptr;                // per-species zigzag scratch (aj layout)
+  void* fold_tmp = nullptr;            // scratch of the guard folds, grown on demand
+  int64_t fold_tmp_bytes = 0;
   emsesg_counter* d_counter = nullptr;
   double* d_randoms = nullptr;
   int64_t n_randoms = 0;
@@ -279,6 +281,8 @@ int exclusive_scan_u32(emsesg_ctx* ctx, uint32_t* data, int64_t n);
 int exclusive_scan_i64(emsesg_ctx* ctx, int64_t* data, int64_t n);
 int ensure_sort_scratch(emsesg_ctx* ctx, int64_t n);
 
+// Scratch of at least `bytes` for the guard folds (kept with the context).
+int fold_scratch(emsesg_ctx* ctx, int64_t bytes, void** out);
 int fx_alloc(emsesg_ctx* ctx);
 void fx_free(emsesg_ctx* ctx);
 void es_free(emsesg_ctx* ctx);

@@ -83,6 +83,19 @@ void timer_collect(emsesg_ctx* ctx) {
   ctx->timer.pending.clear();
 }
 
+int fold_scratch(emsesg_ctx* ctx, int64_t bytes, void** out) {
+  if (ctx->fold_tmp_bytes < bytes) {
+    EMSESG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    cudaFree(ctx->fold_tmp);
+    ctx->fold_tmp = nullptr;
+    ctx->fold_tmp_bytes = 0;
+    EMSESG_CUDA(ctx, cudaMalloc(&ctx->fold_tmp, (size_t)bytes));
+    ctx->fold_tmp_bytes = bytes;
+  }
+  *out = ctx->fold_tmp;
+  return EMSESG_OK;
+}
+
 }  // namespace emsesg
 
 using namespace emsesg;
@@ -177,6 +190,7 @@ extern "C" int emsesg_destroy(emsesg_ctx* ctx) {
   for (int f = 0; f < EMSESG_NFIELDS; f++) cudaFree(ctx->field[f]);
   cudaFree(ctx->node64);
   cudaFree(ctx->tj);
+  cudaFree(ctx->fold_tmp);
   cudaFree(ctx->d_counter);
   cudaFree(ctx->d_count);
   cudaFree(ctx->d_randoms);

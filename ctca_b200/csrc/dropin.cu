@@ -10,7 +10,7 @@
 #include <cstring>
 
 #include "common.cuh"
-#include "slab.cuh"
+#include "fold_point.cuh"
 
 namespace emsesg {
 
@@ -1172,9 +1172,8 @@ extern "C" int emsesg_reduce_rho(emsesg_ctx* ctx, int field) {
     return set_error(ctx, EMSESG_ERR_ARG, "reduce_rho takes a rho-type field");
   FieldDesc f = field_desc(ctx->cfg, field);
   int narr = field == EMSESG_FIELD_RHOBKSP ? ctx->cfg.nspec : 1;
-  std::vector<SlabOp> ops = fold_ops(ctx->cfg, 0, f.nc);
   for (int a = 0; a < narr; a++) {
-    int rc = run_slab_ops(ctx, ctx->field[field] + (int64_t)a * f.size(), f, ops, "reduce_rho");
+    int rc = run_fold(ctx, ctx->field[field] + (int64_t)a * f.size(), f, 0, "reduce_rho");
     if (rc) return rc;
   }
   return EMSESG_OK;
@@ -1182,14 +1181,12 @@ extern "C" int emsesg_reduce_rho(emsesg_ctx* ctx, int field) {
 
 extern "C" int emsesg_reduce_aj(emsesg_ctx* ctx) {
   if (!ctx) return EMSESG_ERR_ARG;
-  FieldDesc f = field_desc(ctx->cfg, EMSESG_FIELD_AJ);
-  return run_slab_ops(ctx, ctx->field[EMSESG_FIELD_AJ], f, fold_ops(ctx->cfg, 1, 3), "reduce_aj");
+  return run_fold(ctx, ctx->field[EMSESG_FIELD_AJ], field_desc(ctx->cfg, EMSESG_FIELD_AJ), 1, "reduce_aj");
 }
 
 extern "C" int emsesg_reduce_ajdg(emsesg_ctx* ctx) {
   if (!ctx) return EMSESG_ERR_ARG;
-  FieldDesc f = field_desc(ctx->cfg, EMSESG_FIELD_AJDG);
-  return run_slab_ops(ctx, ctx->field[EMSESG_FIELD_AJDG], f, fold_ops(ctx->cfg, 1, f.nc), "reduce_ajdg");
+  return run_fold(ctx, ctx->field[EMSESG_FIELD_AJDG], field_desc(ctx->cfg, EMSESG_FIELD_AJDG), 1, "reduce_ajdg");
 }
 
 extern "C" int emsesg_rhoupd(emsesg_ctx* ctx, int ps) {
@@ -1230,7 +1227,7 @@ extern "C" int emsesg_exchange_eb(emsesg_ctx* ctx) {
   int rc = apply_pending_eb(ctx);
   if (rc) return rc;
   const FieldDesc f = field_desc(ctx->cfg, EMSESG_FIELD_EB);
-  return run_slab_ops(ctx, ctx->field[EMSESG_FIELD_EB], f, fold_ops(ctx->cfg, 2, 6), "exchange_eb");
+  return run_fold(ctx, ctx->field[EMSESG_FIELD_EB], f, 2, "exchange_eb");
 }
 
 extern "C" int emsesg_energy(emsesg_ctx* ctx, double* engk) {
