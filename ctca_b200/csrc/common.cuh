@@ -87,6 +87,9 @@ struct FxState {
   int64_t* tile_start = nullptr;    // [nspec][ntiles+1] sorted ranks of each tile's first particle
   int64_t* tile_pad = nullptr;      // [nspec][ntiles+1] first slot of each tile's padded region
   int64_t* chunk_start = nullptr;   // [nspec][ntiles+1] first push CTA of each tile
+  void* chunks = nullptr;           // [nspec][nchunk_max] the push's row chunks (int4: tile, rows, slot)
+  int64_t nchunk_max = 0;           // one chunk a row at most
+  bool chunks_stale = true;         // chunk_start and chunks are not of the present tile_start (the sort keeps it)
   int64_t base[EMSESG_ISPEC] = {};  // species region offsets in pos / vx / vy / vz
   int64_t cap[EMSESG_ISPEC] = {};   // species region sizes (capacity + tile padding)
   bool tiled = false;               // regions hold the thread-major layout of a sort
@@ -99,7 +102,9 @@ struct FxState {
   uint32_t* lcs_wcnt = nullptr;     // [ntiles][warps][nbc] of the species being sorted
   uint32_t* lcs_celltot = nullptr;  // [ntiles][tile cells]
   int64_t* lcs_tiletot = nullptr;   // [ntiles]
-  int* lcs_stray = nullptr;         // [nspec]
+  int* lcs_stray = nullptr;         // [ISPEC] more strays than the tile sort takes, [ISPEC] strays
+  unsigned long long* lcs_slist = nullptr;  // [STRAY_MAX] strays of the species being sorted: cell key, slot
+  uint32_t* lcs_regend = nullptr;   // [ntiles][tile cells] first rank of a cell's strays
   uint32_t* lcs_inv = nullptr;      // per slot: the old slot of its particle
   // box bodies: absorbed minus emitted particles per surface cell
   unsigned long long* surf = nullptr;  // [nspec][nsurf]
@@ -140,7 +145,9 @@ struct FxState {
   AdjWork* adj = nullptr;
   uint32_t* defer = nullptr;        // one bit per slot: left for k_fx_deferred by the parts of a step
   int64_t defer_words = 0;
-  int64_t* accum = nullptr;         // int64 (rho, jx, jy, jz) on the rho layout
+  int64_t* accum = nullptr;         // int64 rho (rho layout), then J (aj layout), as the push left them
+  int64_t* accum_mem = nullptr;     // its allocation: two words before it (the continuity maxima), cleared with it
+  bool fold_rho = false, fold_j = false;  // guard folds of accum not done in place (the fields have them)
   double* diag = nullptr;           // FP64 checks: energy partials, sums, continuity maxima
   bool rho_prev = false;            // the rho field holds the deposit of the step before
   bool cont_valid = false;          // ... so the last step's continuity residual is meaningful

@@ -29,6 +29,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "fold_point.cuh"
 #include "slab.cuh"
 
 namespace emsesg {
@@ -36,6 +37,7 @@ namespace emsesg {
 namespace {
 
 constexpr uint32_t DEAD = 0xFFFFFFFFu;
+constexpr int ACCUM_PAD = 2;  // words before the accumulators: the continuity maxima
 constexpr double FIX_INV = 1.0 / 1099511627776.0;
 
 struct Geo {
@@ -52,6 +54,15 @@ __device__ __forceinline__ void unpack(const Geo& g, uint32_t c, int& i, int& j,
 }
 __device__ __forceinline__ uint32_t pack(const Geo& g, int i, int j, int k) {
   return (uint32_t)i | ((uint32_t)j << g.bx) | ((uint32_t)k << (g.bx + g.by));
+}
+
+// Tile-major cell key of a cell.
+__device__ __forceinline__ uint32_t cell_key(const Geo& g, int i, int j, int k) {
+  const uint32_t tile = (uint32_t)(i / g.t[0]) +
+                        (uint32_t)g.nt[0] * ((uint32_t)(j / g.t[1]) + (uint32_t)g.nt[1] * (uint32_t)(k / g.t[2]));
+  const uint32_t in = (uint32_t)(i % g.t[0]) +
+                      (uint32_t)g.t[0] * ((uint32_t)(j % g.t[1]) + (uint32_t)g.t[1] * (uint32_t)(k % g.t[2]));
+  return tile * (uint32_t)(g.t[0] * g.t[1] * g.t[2]) + in;
 }
 
 // ---------------------------------------------------------------- fields
@@ -81,13 +92,6 @@ __global__ void k_grdcrt32(const double* __restrict__ eb, float4* __restrict__ f
 
 // ---------------------------------------------------------------- push
 #include "fx_push.cuh"
-
-// int64 fixed point -> FP64 field (scale 2^-40).
-__global__ void k_fix_to_double(const long long* __restrict__ src, double* __restrict__ dst, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  dst[i] = (double)src[i] * FIX_INV;
-}
 
 // ---------------------------------------------------------------- load / store / sort
 // (cell, offset) of one FP64 coordinate.  An offset that rounds up to 1.0f,
@@ -235,10 +239,7 @@ __global__ void k_fx_keys(const float4* __restrict__ pos, int64_t n, const int64
     if (cell != DEAD) {
       int i, j, k;
       unpack(g, cell, i, j, k);
-      uint32_t tile = (uint32_t)(i / g.t[0]) +
-                      (uint32_t)g.nt[0] * ((uint32_t)(j / g.t[1]) + (uint32_t)g.nt[1] * (uint32_t)(k / g.t[2]));
-      uint32_t in = (uint32_t)(i % g.t[0]) + (uint32_t)g.t[0] * ((uint32_t)(j % g.t[1]) + (uint32_t)g.t[1] * (uint32_t)(k % g.t[2]));
-      key = tile * (uint32_t)(g.t[0] * g.t[1] * g.t[2]) + in;
+      key = cell_key(g, i, j, k);
     }
   }
   keys[m] = key;
@@ -491,14 +492,18 @@ int fx_alloc(emsesg_ctx* ctx) {
   EMSESG_CUDA(ctx, cudaMalloc(&f.tile_pad, (int64_t)c.nspec * (f.ntiles + 1) * sizeof(int64_t)));
   EMSESG_CUDA(ctx, cudaMalloc(&f.chunk_start, (int64_t)c.nspec * (f.ntiles + 1) * sizeof(int64_t)));
   FieldDesc fr = field_desc(c, EMSESG_FIELD_RHO), fj = field_desc(c, EMSESG_FIELD_AJ);
-  EMSESG_CUDA(ctx, cudaMalloc(&f.accum, (fr.size() + fj.size()) * sizeof(int64_t)));
+  EMSESG_CUDA(ctx, cudaMalloc(&f.accum_mem, (ACCUM_PAD + fr.size() + fj.size()) * sizeof(int64_t)));
+  EMSESG_CUDA(ctx, cudaMemsetAsync(f.accum_mem, 0, ACCUM_PAD * sizeof(int64_t), ctx->stream));
+  f.accum = f.accum_mem + ACCUM_PAD;
+  for (int is = 0; is < c.nspec; is++) f.nchunk_max = std::max(f.nchunk_max, f.tail0[is] / PUSH_THREADS + 1);
+  EMSESG_CUDA(ctx, cudaMalloc(&f.chunks, (int64_t)c.nspec * f.nchunk_max * sizeof(int4)));
   // one bit per slot: the particles the parts of a step leave for k_fx_deferred
   f.defer_words = (cap + 31) / 32;
   EMSESG_CUDA(ctx, cudaMalloc(&f.defer, f.defer_words * sizeof(uint32_t)));
   EMSESG_CUDA(ctx, cudaMemsetAsync(f.defer, 0, f.defer_words * sizeof(uint32_t), ctx->stream));
-  // FP64 checks: energy partials and sums, the continuity maxima
-  EMSESG_CUDA(ctx, cudaMalloc(&f.diag, (3 * DIAG_GRID + 3 + 2) * sizeof(double)));
-  EMSESG_CUDA(ctx, cudaMemsetAsync(f.diag, 0, (3 * DIAG_GRID + 3 + 2) * sizeof(double), ctx->stream));
+  // FP64 checks: energy partials and sums
+  EMSESG_CUDA(ctx, cudaMalloc(&f.diag, (3 * DIAG_GRID + 3) * sizeof(double)));
+  EMSESG_CUDA(ctx, cudaMemsetAsync(f.diag, 0, (3 * DIAG_GRID + 3) * sizeof(double), ctx->stream));
   int64_t nn = (int64_t)(c.nx + 1) * (c.ny + 1) * (c.nz + 1);
   EMSESG_CUDA(ctx, cudaMalloc(&f.fnode, nn * sizeof(float4)));
   EMSESG_CUDA(ctx, cudaMalloc(&f.fnode2, nn * sizeof(float4)));
@@ -514,7 +519,11 @@ int fx_alloc(emsesg_ctx* ctx) {
     EMSESG_CUDA(ctx, cudaMalloc(&f.lcs_wcnt, f.ntiles * PUSH_WARPS * nbc * sizeof(uint32_t)));  // one species
     EMSESG_CUDA(ctx, cudaMalloc(&f.lcs_celltot, f.ntiles * tcells * sizeof(uint32_t)));
     EMSESG_CUDA(ctx, cudaMalloc(&f.lcs_tiletot, f.ntiles * sizeof(int64_t)));
-    EMSESG_CUDA(ctx, cudaMalloc(&f.lcs_stray, EMSESG_ISPEC * sizeof(int)));
+    EMSESG_CUDA(ctx, cudaMalloc(&f.lcs_stray, 2 * EMSESG_ISPEC * sizeof(int)));
+    EMSESG_CUDA(ctx, cudaMalloc(&f.lcs_slist, STRAY_MAX * sizeof(unsigned long long)));
+    EMSESG_CUDA(ctx, cudaMalloc(&f.lcs_regend, f.ntiles * tcells * sizeof(uint32_t)));
+    EMSESG_CUDA(ctx, cudaFuncSetAttribute(k_lcs_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)(STRAY_MAX * sizeof(unsigned long long))));
     EMSESG_CUDA(ctx, cudaMalloc(&f.lcs_inv, cap * sizeof(uint32_t)));
     // kernel attributes hold for every context of the process: allow the
     // largest box (8-cell tiles), whatever this context's tile
@@ -546,12 +555,13 @@ void fx_free(emsesg_ctx* ctx) {
   FxState& f = ctx->fx;
   cudaFree(f.pos); cudaFree(f.vx); cudaFree(f.vy); cudaFree(f.vz);
   cudaFree(f.pos2); cudaFree(f.vx2); cudaFree(f.vy2); cudaFree(f.vz2);
-  cudaFree(f.count_d); cudaFree(f.slots_d); cudaFree(f.tile_start); cudaFree(f.tile_pad); cudaFree(f.accum);
-  cudaFree(f.chunk_start); cudaFree(f.defer);
+  cudaFree(f.count_d); cudaFree(f.slots_d); cudaFree(f.tile_start); cudaFree(f.tile_pad); cudaFree(f.accum_mem);
+  cudaFree(f.chunk_start); cudaFree(f.chunks); cudaFree(f.defer);
   cudaFree(f.fnode); cudaFree(f.fnode2);
   cudaFree(f.diag);
   cudaFree(f.tile_start2); cudaFree(f.tile_pad2); cudaFree(f.lcs_cnt); cudaFree(f.lcs_base); cudaFree(f.lcs_wcnt);
   cudaFree(f.lcs_celltot); cudaFree(f.lcs_tiletot); cudaFree(f.lcs_stray); cudaFree(f.lcs_inv);
+  cudaFree(f.lcs_slist); cudaFree(f.lcs_regend);
   cudaFree(f.surf); cudaFree(f.tailord); cudaFree(f.stage); cudaFree(f.stage_ord);
   cudaFreeHost(f.ord_host);
   if (f.ord_ev) cudaEventDestroy(f.ord_ev);
@@ -580,6 +590,7 @@ int64_t sort_slots(emsesg_ctx* ctx, int is) {
 int fx_local_sort(emsesg_ctx* ctx, bool* done) {
   *done = false;
   FxState& f = ctx->fx;
+  f.chunks_stale = true;  // until every species is through
   const emsesg_config& c = ctx->cfg;
   Geo g = make_geo(ctx);
   LcsGeo G[EMSESG_ISPEC] = {};
@@ -613,13 +624,14 @@ int fx_local_sort(emsesg_ctx* ctx, bool* done) {
       if (rc) return rc;
     }
   }
-  EMSESG_CUDA(ctx, cudaMemsetAsync(f.lcs_stray, 0, EMSESG_ISPEC * sizeof(int), ctx->stream));
+  EMSESG_CUDA(ctx, cudaMemsetAsync(f.lcs_stray, 0, 2 * EMSESG_ISPEC * sizeof(int), ctx->stream));
   for (int is = 0; is < c.nspec; is++) {
     int64_t* ts2 = f.tile_start2 + is * T1;
     int64_t* tp2 = f.tile_pad2 + is * T1;
     if (ctx->totalp[is] == 0) {
       EMSESG_CUDA(ctx, cudaMemsetAsync(ts2, 0, T1 * sizeof(int64_t), ctx->stream));
       EMSESG_CUDA(ctx, cudaMemsetAsync(tp2, 0, T1 * sizeof(int64_t), ctx->stream));
+      EMSESG_CUDA(ctx, cudaMemsetAsync(f.chunk_start + is * T1, 0, T1 * sizeof(int64_t), ctx->stream));
       EMSESG_CUDA(ctx, cudaMemsetAsync(f.count_d + is, 0, sizeof(int64_t), ctx->stream));
       EMSESG_CUDA(ctx, cudaMemsetAsync(f.slots_d + is, 0, sizeof(int64_t), ctx->stream));
       continue;
@@ -628,13 +640,15 @@ int fx_local_sort(emsesg_ctx* ctx, bool* done) {
     uint32_t* cnt = f.lcs_cnt + is * f.ntiles * nbc;
     uint32_t* bas = f.lcs_base + is * f.ntiles * nbc;
     const int* stray = f.lcs_stray + is;
+    int* nstray = f.lcs_stray + EMSESG_ISPEC + is;
     // per-warp counts (one species at a time)
     EMSESG_LAUNCH(ctx, "lcs_count", k_lcs_count, (unsigned)f.ntiles, PUSH_THREADS, lsm, f.pos + off,
-                  f.tile_start + is * T1, f.tile_pad + is * T1, g, G[is], f.lcs_wcnt, cnt, f.lcs_stray + is);
-    // Outside a stream capture the host reads the stray flag and falls back
-    // to the radix sort (which redoes every species).  Inside one
-    // (emsesg_fx_run's graph) it cannot: the sort kernels of a species with
-    // a stray then return at once and k_lcs_keep carries its current order
+                  f.tile_start + is * T1, f.tile_pad + is * T1, g, G[is], f.lcs_wcnt, cnt, f.lcs_stray + is, nstray,
+                  f.lcs_slist);
+    // Outside a stream capture the host reads the flag of too many strays and
+    // falls back to the radix sort (which redoes every species).  Inside one
+    // (emsesg_fx_run's graph) it cannot: the sort kernels of such a species
+    // then return at once and k_lcs_keep carries its current order
     // over to the new buffers.
     if (!f.capture) {
       int st = 0;
@@ -656,13 +670,16 @@ int fx_local_sort(emsesg_ctx* ctx, bool* done) {
     if (nt > 0)
       EMSESG_LAUNCH(ctx, "lcs_tail_count", k_lcs_tail_count, nblk(nt), 256, 0, tk, nt, deadkey, (int)tcells,
                     f.lcs_celltot, (unsigned long long*)f.lcs_tiletot, stray);
-    EMSESG_LAUNCH(ctx, "lcs_tiles", k_lcs_tiles, 1, 1024, 0, f.lcs_tiletot, f.ntiles, ts2, tp2, f.count_d + is,
-                  f.slots_d + is, stray);
+    EMSESG_LAUNCH(ctx, "lcs_tiles", k_lcs_tiles, 1, 1024, STRAY_MAX * sizeof(unsigned long long), f.lcs_tiletot,
+                  f.lcs_celltot, f.ntiles, ts2, tp2, f.chunk_start + is * T1,
+                  (int4*)f.chunks + is * f.nchunk_max, f.chunk_rows, f.count_d + is,
+                  f.slots_d + is, stray, nstray, f.lcs_slist, (int)tcells);
     EMSESG_LAUNCH(ctx, "lcs_bases", k_lcs_bases, (unsigned)f.ntiles, CELL_THREADS, 0, cnt, f.lcs_celltot, g, G[is],
-                  ts2, tp2, bas, f.lcs_inv + off, stray);
+                  ts2, tp2, bas, f.lcs_inv + off, stray, nstray, f.lcs_regend);
     EMSESG_LAUNCH(ctx, "lcs_rank", k_lcs_rank, (unsigned)f.ntiles, PUSH_THREADS, lsm, f.pos + off,
                   f.tile_start + is * T1, f.tile_pad + is * T1, g, G[is], f.lcs_wcnt,
-                  bas, ts2, tp2, f.lcs_inv + off, ctx->d_status, ctx->d_diag, stray);
+                  bas, ts2, tp2, f.lcs_inv + off, ctx->d_status, ctx->d_diag, stray, nstray, f.lcs_slist,
+                  f.lcs_regend);
     if (nt > 0)
       EMSESG_LAUNCH(ctx, "lcs_tail_inv", k_lcs_tail_inv, nblk(nt), 256, 0, tk, tv, nt, deadkey, (int)tcells,
                     f.lcs_celltot, ts2, tp2, f.lcs_inv + off, stray);
@@ -692,6 +709,7 @@ int fx_local_sort(emsesg_ctx* ctx, bool* done) {
   std::swap(f.tile_start, f.tile_start2);
   std::swap(f.tile_pad, f.tile_pad2);
   for (int is = 0; is < c.nspec; is++) f.ntail[is] = 0;  // merged into the regions
+  f.chunks_stale = false;
   *done = true;
   return EMSESG_OK;
 }
@@ -748,6 +766,7 @@ extern "C" int emsesg_fx_sort(emsesg_ctx* ctx) {
   std::swap(f.vy, f.vy2);
   std::swap(f.vz, f.vz2);
   f.tiled = true;
+  f.chunks_stale = true;
   return EMSESG_OK;
 }
 
@@ -1051,8 +1070,12 @@ int fx_push_phase(emsesg_ctx* ctx, int ustep, bool deposit, bool jd) {
   // step without the current (jd false) leaves J's accumulator alone.
   if (deposit) {
     const int64_t nz = fr.size() + (jd && !f.inj_j_pending ? fj.size() : 0);
-    EMSESG_CUDA(ctx, cudaMemsetAsync(f.accum, 0, nz * sizeof(int64_t), ctx->stream));
-    if (jd) f.inj_j_pending = false;
+    EMSESG_CUDA(ctx, cudaMemsetAsync(f.accum_mem, 0, (ACCUM_PAD + nz) * sizeof(int64_t), ctx->stream));
+    f.fold_rho = false;
+    if (jd) {
+      f.inj_j_pending = false;
+      f.fold_j = false;
+    }
   }
   int tmax = std::max(f.tile[0], std::max(f.tile[1], f.tile[2]));
   int smem = fx_push_smem(tmax, !deposit || jd);
@@ -1062,11 +1085,10 @@ int fx_push_phase(emsesg_ctx* ctx, int ustep, bool deposit, bool jd) {
   if (!deposit && f.move_src.pos) {
     a.rpos = f.move_src.pos; a.rvx = f.move_src.vx; a.rvy = f.move_src.vy; a.rvz = f.move_src.vz;
   }
-  a.tile_start = f.tile_start;
-  a.tile_pad = f.tile_pad;
   a.chunk_start = f.chunk_start;
+  a.chunks = (const int4*)f.chunks;
+  a.nchunk_max = f.nchunk_max;
   a.ntiles = f.ntiles;
-  a.chunk_rows = f.chunk_rows;
   double gustep = ustep;
   a.gustep = (float)gustep;
   a.rustep = (float)(1.0 / ustep);
@@ -1092,20 +1114,23 @@ int fx_push_phase(emsesg_ctx* ctx, int ustep, bool deposit, bool jd) {
     EMSESG_CUDA(ctx, cudaMemsetAsync(f.outbox_n, 0, 2 * EMSESG_ISPEC * sizeof(unsigned long long), ctx->stream));
     a.ob = Outbox{f.outbox, f.outbox_n, f.outbox_cap};
   }
+  if (f.chunks_stale) {
+    EMSESG_LAUNCH(ctx, "fx_chunks", k_push_chunks, (unsigned)c.nspec, 1024, 0, f.tile_start, f.tile_pad, f.ntiles,
+                  f.chunk_start, (int4*)f.chunks, f.nchunk_max, f.chunk_rows);
+    f.chunks_stale = false;
+  }
   // row chunks of the tile regions: at most ntiles + rows / chunk_rows
   int64_t rows = 0;
   for (int is = 0; is < c.nspec; is++) rows = std::max(rows, (f.cap[is] + PUSH_THREADS - 1) / PUSH_THREADS);
-  EMSESG_LAUNCH(ctx, "fx_chunks", k_push_chunks, (unsigned)c.nspec, 1024, 0, f.tile_start, f.ntiles, f.chunk_start,
-                f.chunk_rows);
   dim3 grid((unsigned)(f.ntiles + rows / f.chunk_rows + 1), (unsigned)c.nspec);
   if (!deposit) {
     for (int is = 0; is < c.nspec; is++)
       if (f.ntail[is]) return set_error(ctx, EMSESG_ERR_STATE, "move-only step with injected particles");
     if (a.bd.n > 0) return set_error(ctx, EMSESG_ERR_UNSUPPORTED, "move-only step with bodies");
     if (fx_box_tile(tmax) == 4)
-      EMSESG_LAUNCH(ctx, "fx_move", (k_fx_push<4, false>), grid, PUSH_BLOCK, smem, a);
+      EMSESG_LAUNCH(ctx, "fx_move", (k_fx_push<4, false>), grid, PUSH_THREADS, smem, a);
     else
-      EMSESG_LAUNCH(ctx, "fx_move", (k_fx_push<8, false>), grid, PUSH_BLOCK, smem, a);
+      EMSESG_LAUNCH(ctx, "fx_move", (k_fx_push<8, false>), grid, PUSH_THREADS, smem, a);
     return EMSESG_OK;
   }
   // tile regions next to a body take the general path when a particle can
@@ -1114,7 +1139,7 @@ int fx_push_phase(emsesg_ctx* ctx, int ustep, bool deposit, bool jd) {
   const bool curv = a.bd.ncurved > 0 || f.box_inside;
   const PushKernel kern = push_kernel(fx_box_tile(tmax), curv, jd);
   if (!parts) {
-    EMSESG_LAUNCH(ctx, "fx_push", kern, grid, PUSH_BLOCK, smem, a);
+    EMSESG_LAUNCH(ctx, "fx_push", kern, grid, PUSH_THREADS, smem, a);
   } else {
     const PushKernel pkern = push_kernel(fx_box_tile(tmax), curv, jd, true);
     // part p: the node planes its chunk completes (its tiles' boxes), then
@@ -1133,7 +1158,7 @@ int fx_push_phase(emsesg_ctx* ctx, int ustep, bool deposit, bool jd) {
       ap.t_n = ptile[p + 1] - ptile[p];
       ap.zready = zready[p];
       dim3 pgrid((unsigned)(ap.t_n + rows / f.chunk_rows + 1), (unsigned)c.nspec);
-      EMSESG_LAUNCH(ctx, "fx_push_part", pkern, pgrid, PUSH_BLOCK, smem, ap);
+      EMSESG_LAUNCH(ctx, "fx_push_part", pkern, pgrid, PUSH_THREADS, smem, ap);
     }
     // the particles the parts left, every node plane converted
     EMSESG_LAUNCH(ctx, "fx_deferred", deferred_kernel(fx_box_tile(tmax), curv, jd), nblk(f.defer_words), 256, 0,
@@ -1156,19 +1181,14 @@ int fx_push_phase(emsesg_ctx* ctx, int ustep, bool deposit, bool jd) {
   return EMSESG_OK;
 }
 
-// The fold lists of rho and J split for slab mode: the border exchange of
-// the x and y axes (run by emsesg_fx_slab_begin, before the ranks exchange
-// their z border planes) and the rest (run by emsesg_fx_slab_end).  Without
-// slab mode the whole lists.
-void fold_lists(const emsesg_config& c, bool slab, int part, std::vector<SlabOp>* rho, std::vector<SlabOp>* j) {
+// The fold lists of rho and J split for slab mode: part 0, the border exchange
+// of the x and y axes (run by emsesg_fx_slab_border, before the ranks exchange
+// their z border planes), and part 1, the folds (run by emsesg_fx_slab_end).
+void fold_lists(const emsesg_config& c, int part, std::vector<SlabOp>* rho, std::vector<SlabOp>* j) {
   for (int kind = 0; kind < 2; kind++) {
     std::vector<SlabOp> all = fold_ops(c, kind, kind == 0 ? 1 : 3);
     std::vector<SlabOp>& out = kind == 0 ? *rho : *j;
     out.clear();
-    if (!slab) {
-      out = all;
-      continue;
-    }
     int nex = 0;  // the exchange copies come first, two per periodic axis
     for (int d = 0; d < 3; d++)
       if (c.nfbnd[d] == 0) nex += 2;
@@ -1181,31 +1201,47 @@ void fold_lists(const emsesg_config& c, bool slab, int part, std::vector<SlabOp>
 }
 
 // The rest of a step after its push (and, in slab mode, the exchange of the
-// z border planes and the arrivals): guard folds on the exact integers,
-// FP64 rho and J (J first: the conversion of rho takes the continuity
-// residual of the step against the rho field of the step before, still in
-// place, and this J), then the re-sort after the push (so that injected
-// particles take their first, partial step before they join the tile
-// regions).
+// z border planes and the arrivals): guard folds on the exact integers and
+// FP64 J and rho with the continuity residual (k_fx_j, k_fx_rho), then the re-sort
+// after the push (so that injected particles take their first, partial step
+// before they join the tile regions).
 int fx_fields_phase(emsesg_ctx* ctx, bool jd) {
   FxState& f = ctx->fx;
   const emsesg_config& c = ctx->cfg;
-  FieldDesc fr = field_desc(c, EMSESG_FIELD_RHO), fj = field_desc(c, EMSESG_FIELD_AJ);
-  unsigned long long* acc_rho = (unsigned long long*)f.accum;
-  unsigned long long* acc_j = acc_rho + fr.size();
-  std::vector<SlabOp> orho, oj;
-  fold_lists(c, f.slab, 1, &orho, &oj);
-  if (!jd) oj.clear();
-  int rc;
-  if ((rc = run_slab_ops2(ctx, (long long*)acc_rho, fr, orho, (long long*)acc_j, fj, oj, "fx_fold"))) return rc;
-  if (jd)
-    EMSESG_LAUNCH(ctx, "fx_to_double", k_fix_to_double, nblk(fj.size()), 256, 0, (const long long*)acc_j,
-                  ctx->field[EMSESG_FIELD_AJ], fj.size());
-  unsigned long long* cres = (unsigned long long*)(f.diag + 3 * DIAG_GRID + 3);
-  EMSESG_CUDA(ctx, cudaMemsetAsync(cres, 0, 2 * sizeof(double), ctx->stream));
-  EMSESG_LAUNCH(ctx, "fx_to_double", k_fix_to_rho, nblk(fr.size(), RHO_BLOCK), RHO_BLOCK, 0, (const long long*)acc_rho,
-                ctx->field[EMSESG_FIELD_RHO], jd ? ctx->field[EMSESG_FIELD_AJ] : nullptr, fr, fj, c.nx, c.ny, c.nz,
-                cres);
+  const FieldDesc fr = field_desc(c, EMSESG_FIELD_RHO), fj = field_desc(c, EMSESG_FIELD_AJ);
+  if (f.slab) {
+    // the copies of x and y are in the accumulators, those of z come from the
+    // ranks: the folds alone, in place
+    std::vector<SlabOp> orho, oj;
+    fold_lists(c, 1, &orho, &oj);
+    int rc = run_slab_ops2(ctx, (long long*)f.accum, fr, orho, (long long*)f.accum + fr.size(), fj, oj, "fx_fold");
+    if (rc) return rc;
+  } else {
+    f.fold_rho = true;
+    if (jd) f.fold_j = true;
+  }
+  FieldsArgs a{};
+  a.fj = fj;
+  a.fold = !f.slab;
+  a.res = (unsigned long long*)f.accum_mem;
+  const bool wide = fj.size() + FIELD_BLOCK * FIELD_VEC >= (1LL << 32);
+  if (jd) {
+    a.acc = (const long long*)f.accum + fr.size();
+    a.out = ctx->field[EMSESG_FIELD_AJ];
+    a.f = fj;
+    a.g = fold_geo(c, 1);
+    a.shell = fold_shell(fj);
+    a.blocks = nblk(fj.size(), FIELD_BLOCK * FIELD_VEC);
+    const unsigned sb = a.fold ? nblk((a.shell.nzs + a.shell.nys + a.shell.nxs) * fj.nc, FIELD_BLOCK) : 0;
+    EMSESG_LAUNCH(ctx, "fx_j", (wide ? k_fx_j<int64_t> : k_fx_j<uint32_t>), a.blocks + sb, FIELD_BLOCK, 0, a);
+  }
+  a.acc = (const long long*)f.accum;
+  a.out = ctx->field[EMSESG_FIELD_RHO];
+  a.aj = jd ? ctx->field[EMSESG_FIELD_AJ] : nullptr;
+  a.f = fr;
+  a.g = fold_geo(c, 0);
+  EMSESG_LAUNCH(ctx, "fx_rho", (wide ? k_fx_rho<int64_t> : k_fx_rho<uint32_t>), nblk(fr.size(), FIELD_BLOCK), FIELD_BLOCK,
+                0, a);
   // the continuity residual needs the step's current
   f.cont_valid = jd && f.rho_prev;
   f.rho_prev = true;
@@ -1696,6 +1732,7 @@ extern "C" int emsesg_fx_chunk_rows(emsesg_ctx* ctx, int rows) {
     f.gexec = nullptr;
   }
   f.chunk_rows = rows;
+  f.chunks_stale = true;
   return EMSESG_OK;
 }
 
@@ -1819,7 +1856,7 @@ extern "C" int emsesg_fx_slab_border(emsesg_ctx* ctx) {
   FieldDesc fr = field_desc(c, EMSESG_FIELD_RHO), fj = field_desc(c, EMSESG_FIELD_AJ);
   unsigned long long* acc_rho = (unsigned long long*)f.accum;
   std::vector<SlabOp> orho, oj;
-  fold_lists(c, true, 0, &orho, &oj);
+  fold_lists(c, 0, &orho, &oj);
   int rc = run_slab_ops2(ctx, (long long*)acc_rho, fr, orho, (long long*)(acc_rho + fr.size()), fj, oj, "fx_fold");
   if (rc) return rc;
   return emsesg_synchronize(ctx);
@@ -1951,6 +1988,7 @@ int inflow_impl(emsesg_ctx* ctx, int spec, int axis, int front, int64_t n, const
     if (!f.inj_j_pending) {
       EMSESG_CUDA(ctx, cudaMemsetAsync(cur.acc, 0, cur.fj.size() * sizeof(int64_t), ctx->stream));
       f.inj_j_pending = true;
+      f.fold_j = false;
     }
     cur.qfix = c.q[is] * 1099511627776.0;
     cur.ustep = ustep;
@@ -2023,7 +2061,7 @@ extern "C" int emsesg_fx_continuity(emsesg_ctx* ctx, double* res) {
   if (!ctx->fx.loaded) return set_error(ctx, EMSESG_ERR_STATE, "FP32 form not loaded");
   FxState& f = ctx->fx;
   double r[2];
-  EMSESG_CUDA(ctx, cudaMemcpyAsync(r, f.diag + 3 * DIAG_GRID + 3, sizeof(r), cudaMemcpyDeviceToHost, ctx->stream));
+  EMSESG_CUDA(ctx, cudaMemcpyAsync(r, f.accum_mem, sizeof(r), cudaMemcpyDeviceToHost, ctx->stream));
   EMSESG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   res[0] = f.cont_valid ? r[0] : std::nan("");
   res[1] = f.rho_prev ? r[1] : std::nan("");
@@ -2056,6 +2094,16 @@ extern "C" int emsesg_fx_download_accum(emsesg_ctx* ctx, int64_t* host) {
   if (!ctx || !host) return EMSESG_ERR_ARG;
   if (!ctx->fx.accum) return set_error(ctx, EMSESG_ERR_STATE, "FP32 form not loaded");
   FieldDesc fr = field_desc(ctx->cfg, EMSESG_FIELD_RHO), fj = field_desc(ctx->cfg, EMSESG_FIELD_AJ);
+  // the step folds while it converts (k_fx_j, k_fx_rho); the integers are folded
+  // in place when they are asked for
+  FxState& f = ctx->fx;
+  if (f.fold_rho || f.fold_j) {
+    int rc = EMSESG_OK;
+    if (f.fold_rho) rc = run_fold(ctx, (long long*)f.accum, fr, 0, "fx_fold");
+    if (!rc && f.fold_j) rc = run_fold(ctx, (long long*)f.accum + fr.size(), fj, 1, "fx_fold");
+    if (rc) return rc;
+    f.fold_rho = f.fold_j = false;
+  }
   EMSESG_CUDA(ctx, cudaMemcpyAsync(host, ctx->fx.accum, (fr.size() + fj.size()) * sizeof(int64_t),
                                    cudaMemcpyDeviceToHost, ctx->stream));
   EMSESG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -2218,6 +2266,7 @@ int snap_copy(emsesg_ctx* ctx, bool save, FxSnap& sn, int64_t cap, int64_t nl, b
   EMSESG_SNAP(sn.counts, f.count_d, EMSESG_ISPEC * sizeof(int64_t));
   EMSESG_SNAP(sn.counts + EMSESG_ISPEC, f.slots_d, EMSESG_ISPEC * sizeof(int64_t));
 #undef EMSESG_SNAP
+  if (!save) f.chunks_stale = true;
   return EMSESG_OK;
 }
 
@@ -2414,6 +2463,7 @@ extern "C" int emsesg_fx_adjoint(emsesg_ctx* ctx, int K, int ustep, int ckpt, in
         const int64_t* t = w.meta[(size_t)ks];
         const cudaMemcpyKind dd = cudaMemcpyDeviceToDevice;
         EMSESG_CUDA(ctx, cudaMemcpyAsync(f.tile_start, t, nl * sizeof(int64_t), dd, ctx->stream));
+        f.chunks_stale = true;
         EMSESG_CUDA(ctx, cudaMemcpyAsync(f.tile_pad, t + nl, nl * sizeof(int64_t), dd, ctx->stream));
         EMSESG_CUDA(ctx, cudaMemcpyAsync(f.count_d, t + 2 * nl, EMSESG_ISPEC * sizeof(int64_t), dd, ctx->stream));
         EMSESG_CUDA(ctx, cudaMemcpyAsync(f.slots_d, t + 2 * nl + EMSESG_ISPEC, EMSESG_ISPEC * sizeof(int64_t), dd,
@@ -2527,12 +2577,19 @@ int capture_steps(emsesg_ctx* ctx, int ustep, int block, int sort_every, cudaGra
   float4* pos0 = f.pos;
   const int64_t* ts0 = f.tile_start;
   const uint64_t rs0 = ctx->rng_stream;
+  const bool fr0 = f.fold_rho, fj0 = f.fold_j;
   ctx->timer.on = false;
   EMSESG_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   f.capture = true;
+  // the graph computes the row chunks itself, for the rows per CTA it is
+  // captured with; they are stale for the steps outside it
+  f.chunks_stale = true;
   int rc = EMSESG_OK;
   for (int s = 0; s < block && !rc; s++) rc = emsesg_fx_step(ctx, ustep, (s + 1) % sort_every == 0);
   f.capture = false;
+  f.chunks_stale = true;
+  f.fold_rho = fr0;  // nothing has run
+  f.fold_j = fj0;
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
   ctx->timer.on = timing;
@@ -2548,6 +2605,12 @@ int capture_steps(emsesg_ctx* ctx, int ustep, int block, int sort_every, cudaGra
   }
   *out = graph;
   return EMSESG_OK;
+}
+
+// The host state of the steps that a graph replay ran.
+void graph_ran(FxState& f) {
+  f.chunks_stale = true;
+  f.fold_rho = f.fold_j = true;
 }
 
 bool graph_ready(const emsesg_ctx* ctx) {
@@ -2599,6 +2662,7 @@ extern "C" int emsesg_fx_run(emsesg_ctx* ctx, int ustep, int nsteps, int sort_ev
   }
   const int nblock = nsteps / block;
   for (int b = 0; b < nblock; b++) EMSESG_CUDA(ctx, cudaGraphLaunch(f.gexec, ctx->stream));
+  graph_ran(f);
   if (ctx->ev_fields) EMSESG_CUDA(ctx, cudaEventRecord(ctx->ev_fields, ctx->stream));
   ctx->rng_stream += (uint64_t)nblock * block;
   for (int s = 0; s < nsteps - nblock * block; s++)
@@ -2731,6 +2795,7 @@ extern "C" int emsesg_batch_launch(emsesg_batch* b, int nrep) {
   for (int r = 0; r < n; r++) {
     EMSESG_CUDA(c0, cudaStreamWaitEvent(b->ctxs[r]->stream, b->done, 0));
     b->ctxs[r]->rng_stream += (uint64_t)nrep * b->block;
+    if (nrep > 0) graph_ran(b->ctxs[r]->fx);
     // the graph's reads of eb are over once the run's stream gets here
     if (b->ctxs[r]->ev_fields) EMSESG_CUDA(c0, cudaEventRecord(b->ctxs[r]->ev_fields, b->ctxs[r]->stream));
   }

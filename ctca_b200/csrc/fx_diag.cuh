@@ -75,32 +75,92 @@ __device__ __forceinline__ void max_nonneg(unsigned long long* p, double v) {
   atomicMax(p, (unsigned long long)__double_as_longlong(v));
 }
 
-// rho (FP64) from the folded int64 accumulator (scale 2^-40), and over the
-// nodes 0..n the continuity residual of the step: res[0] = max |rho_new -
-// rho_old + 2 (div J)|, res[1] = max |rho_new| (rhoupd.F90:41-49 gives
-// rho_old - 2 div J as the prediction of rho_new).  The maxima are taken per
-// block (warp shuffles, then the block's warps) before one atomic per block.
-constexpr int RHO_BLOCK = 256;
-__global__ void __launch_bounds__(RHO_BLOCK) k_fix_to_rho(const long long* __restrict__ acc, double* __restrict__ rho,
-                                                          const double* __restrict__ aj, FieldDesc fr, FieldDesc fj,
-                                                          int nx, int ny, int nz, unsigned long long* res) {
-  __shared__ double wmax[2][RHO_BLOCK / 32];
-  const int64_t e = (int64_t)blockIdx.x * RHO_BLOCK + threadIdx.x;
+// The fields of a step from the raw int64 accumulators (scale 2^-40): J, then
+// rho, each with its guard folds (fold_point: the accumulators stay as the push
+// left them) in the pass that converts it to FP64.  Reading and writing the
+// arrays once bounds it; as in-place slabs and two conversions it was 8
+// launches (13 with faces): 136 us a step at 128^3 and 54 us at 32^3 under
+// per-launch events, 116 and 19 us this way.
+constexpr int FIELD_BLOCK = 256;
+constexpr int FIELD_VEC = 4;
+struct FieldsArgs {
+  const long long* acc;
+  double* out;
+  FieldDesc f, fj;
+  const double* aj;             // rho: the step's J, null without the current
+  FoldGeo g;
+  bool fold;                    // false: the accumulators are folded already (slab mode)
+  unsigned blocks;              // J: blocks of its inner elements
+  FoldShell shell;
+  unsigned long long* res;
+};
+// J: the first blocks convert the elements that no fold writes, FIELD_VEC of
+// a row a thread, the others the shell.  I: the type that holds an index.
+template <class I>
+__global__ void __launch_bounds__(FIELD_BLOCK) k_fx_j(FieldsArgs a) {
+  const FieldDesc& f = a.f;
+  if (blockIdx.x < a.blocks) {
+    const I size = (I)f.size();
+    const I e0 = ((I)blockIdx.x * FIELD_BLOCK + (I)threadIdx.x) * FIELD_VEC;
+    if (e0 >= size) return;
+    long long v[FIELD_VEC];
+#pragma unroll
+    for (int q = 0; q < FIELD_VEC; q++) v[q] = e0 + q < size ? a.acc[e0 + q] : 0;
+    const I row = (I)(f.nc * f.ex);
+    const I r = e0 / row;
+    int x = (int)(e0 - r * row);  // element in its row
+    int k = (int)(r / (I)f.ey), j = (int)(r - (I)k * (I)f.ey);
+    const int xlo = f.nc * (2 - f.lo), xhi = f.nc * (a.g.n[0] - 1 - f.lo);
+#pragma unroll
+    for (int q = 0; q < FIELD_VEC; q++) {
+      const bool inner = x >= xlo && x < xhi && j > 1 - f.lo && j < a.g.n[1] - 1 - f.lo && k > 1 - f.lo &&
+                         k < a.g.n[2] - 1 - f.lo;
+      if (e0 + q < size && (inner || !a.fold)) a.out[e0 + q] = (double)v[q] * FIX_INV;
+      if (++x == (int)row) {
+        x = 0;
+        if (++j == f.ey) {
+          j = 0;
+          k++;
+        }
+      }
+    }
+    return;
+  }
+  const int64_t t = (int64_t)(blockIdx.x - a.blocks) * FIELD_BLOCK + threadIdx.x;
+  if (t >= (a.shell.nzs + a.shell.nys + a.shell.nxs) * f.nc) return;
+  int x[3];
+  shell_node(a.shell, t / f.nc, x);
+  const int c = (int)(t % f.nc), i = x[0] + f.lo, j = x[1] + f.lo, k = x[2] + f.lo;
+  a.out[f.at(c, i, j, k)] = (double)fold_point(a.acc, f, a.g, c, i, j, k) * FIX_INV;
+}
+
+// rho, a node a thread, and over the nodes 0..n the continuity residual of
+// the step: res[0] = max |rho_new - rho_old + 2 (div J)|, res[1] = max
+// |rho_new| (rhoupd.F90:41-49 gives rho_old - 2 div J as the prediction of
+// rho_new; the rho field still holds rho_old).  The maxima are taken per block
+// (warp shuffles, then the block's warps) and go to memory only where they
+// exceed what is there.
+template <class I>
+__global__ void __launch_bounds__(FIELD_BLOCK) k_fx_rho(FieldsArgs a) {
+  __shared__ double wmax[2][FIELD_BLOCK / 32];
+  const FieldDesc& f = a.f;
+  const FieldDesc& fj = a.fj;
+  const I e = (I)blockIdx.x * FIELD_BLOCK + (I)threadIdx.x;
   double r = 0.0, m = 0.0;
-  if (e < fr.size()) {
-    const double v = (double)acc[e] * (1.0 / 1099511627776.0);
-    const int64_t ex = fr.ex, ey = fr.ey;
-    const int i = (int)(e % ex) + fr.lo, j = (int)((e / ex) % ey) + fr.lo, k = (int)(e / (ex * ey)) + fr.lo;
-    if (i >= 0 && j >= 0 && k >= 0 && i <= nx && j <= ny && k <= nz) {
-      if (aj) {  // without the step's current (the electrostatic step) no residual
-        const double div = (aj[fj.at(0, i, j, k)] - aj[fj.at(0, i - 1, j, k)]) +
-                           (aj[fj.at(1, i, j, k)] - aj[fj.at(1, i, j - 1, k)]) +
-                           (aj[fj.at(2, i, j, k)] - aj[fj.at(2, i, j, k - 1)]);
-        r = fabs(v - (rho[e] - div * 2.0));
+  if (e < (I)f.size()) {
+    const I row = e / (I)f.ex, plane = row / (I)f.ey;
+    const int i = (int)(e - row * (I)f.ex) + f.lo, j = (int)(row - plane * (I)f.ey) + f.lo, k = (int)plane + f.lo;
+    const long long raw = a.fold && !fold_inner(a.g, i, j, k) ? fold_point(a.acc, f, a.g, 0, i, j, k) : a.acc[e];
+    const double v = (double)raw * FIX_INV;
+    if (i >= 0 && j >= 0 && k >= 0 && i <= a.g.n[0] && j <= a.g.n[1] && k <= a.g.n[2]) {
+      if (a.aj) {  // without the step's current (the electrostatic step) no residual
+        const int64_t x = fj.at(0, i, j, k), sx = fj.nc, sy = sx * fj.ex, sz = sy * fj.ey;
+        const double div = (a.aj[x] - a.aj[x - sx]) + (a.aj[x + 1] - a.aj[x + 1 - sy]) + (a.aj[x + 2] - a.aj[x + 2 - sz]);
+        r = fabs(v - (a.out[e] - div * 2.0));
       }
       m = fabs(v);
     }
-    rho[e] = v;
+    a.out[e] = v;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -115,8 +175,8 @@ __global__ void __launch_bounds__(RHO_BLOCK) k_fix_to_rho(const long long* __res
   __syncthreads();
   if (threadIdx.x < 2) {
     double v = 0.0;
-    for (int w = 0; w < RHO_BLOCK / 32; w++) v = fmax(v, wmax[threadIdx.x][w]);
-    if (v > 0.0) max_nonneg(&res[threadIdx.x], v);
+    for (int w = 0; w < FIELD_BLOCK / 32; w++) v = fmax(v, wmax[threadIdx.x][w]);
+    if (v > __longlong_as_double(*(volatile long long*)&a.res[threadIdx.x])) max_nonneg(&a.res[threadIdx.x], v);
   }
 }
 

@@ -7,55 +7,65 @@
 // thread t's contiguous run of the cell-sorted order, and row r is one
 // coalesced stretch of PUSH_THREADS records.  Empty slots hold DEAD cells.
 //
-// One CTA pushes one region with 736 threads; a 24th warp streams the rows
-// into a 3-stage shared-memory ring with cp.async.bulk (TMA 1-D copies
-// completing on mbarriers) and never computes, so a warp busy with its
-// queues never holds up the stream; pushing warps release a stage through an
-// "empty" mbarrier once they hold their particle.  The
-// tile's FP32 E/B nodes (tile + 1-cell guard) sit in shared memory.
+// One CTA of 736 threads pushes one row chunk of a region.  Each warp copies
+// its own 32 columns of the rows ahead (cp.async, a ring of three rows a warp),
+// so the warps share no barrier inside the rows.  The tile's FP32 E/B nodes
+// (tile + 1-cell guard) sit in shared memory.
 //
-// Per particle: trilinear gather, Buneman-Boris, move.  A particle that
-// stays inside its cell (the common case) adds its two zigzag segments and
-// its CIC charge to 20 FP32 registers that follow the thread's current cell
-// ("run"); when the run's cell changes the 20 sums go through a per-warp
-// queue and are added, converted to int64 fixed point, into the CTA's tile
-// accumulator by all lanes together.  A particle that stays in its cell
-// but is out of place in the thread's run (it changed cell since the sort)
-// puts its 20 values into the same queue as a one-particle run.  A particle
-// that leaves its cell (or whose cell lies outside the tile box) is appended
-// to a per-warp "cross" queue; when 32 are queued, every lane takes one and
-// runs the general path (per-axis boundary rules, relay point, two segments
-// in different cells, charge at the new cell) with direct int64 atomics.  So
-// the divergent work of the few cell-crossing particles runs with all lanes
-// busy.
+// Per particle: trilinear gather, Buneman-Boris, move.  A particle in its
+// thread's current cell (the "run", the common case) that stays in it adds its
+// two zigzag segments and its CIC charge to 20 FP32 registers; when the run
+// ends the 20 sums go through a per-warp queue and are added, converted to
+// int64 fixed point, into the CTA's tile accumulator by all lanes together.
+// A particle out of place in the thread's run (it changed cell since the
+// sort) goes on a per-warp list, and so does one that leaves its cell; a full
+// batch of a list is taken by the whole warp, a particle a lane: out-of-place
+// ones are kicked, moved and added with shared-memory atomics, crossing ones
+// take the general path (per-axis boundary rules, relay point, two segments in
+// different cells, charge at the new cell).  So the divergent work of the few
+// runs with all lanes busy.
+//
+// What bounds it: issue slots (59 % of them) and shared-memory passes (65 %),
+// with the latency of 23 warps a SM between them; DRAM is at 35 %.  At 128^3 x
+// 2 x 64 ppc a push took 7.45 ms with scalar FP32, out-of-place particles in
+// the run queue and rows by bulk copies on shared mbarriers (539 warp
+// instructions a row of 32); 6.81 ms with packed FP32 (f32x2), the
+// interpolation by lerps and the out-of-place list (455); 6.47 ms with rows
+// per warp, 32-bit slot indices and the field rows padded against bank
+// conflicts; 6.29 ms with the chunk table in place of a binary search (2.39
+// TB/s at 56 B a particle).  Not kept, at the same size: rows prefetched in
+// registers (spills, 6.61 ms), the lists out of line (12 ms: generic addresses
+// and an array argument in local memory), all lists at the end of the chunk
+// (7.23 ms: their load latency then meets no other work), a persistent CTA that
+// fetches the next tile during the flush (6.46 ms, and 12 % slower where the
+// push runs in parts).
 //
 // Determinism: a run's FP32 partial sums follow the thread's fixed order;
 // every conversion to fixed point is of one value; integer atomics commute.
 // Two runs on the same input give the same bits.
 
-// 23 pushing warps + 1 streaming warp: 24 warps, 6 on each SM sub-partition,
-// at 80 registers a thread (a few values spill).  The kernel is bound by
-// latency more than by issue or memory: at 128^3 x 64 ppc it pushed in
-// 8.16 ms with 480-slot rows (16 warps, 128 registers), 7.53 with 608 (20
-// warps, 96 registers), 7.20 with 736.
+// 23 warps, 6 on each SM sub-partition, at 80 registers a thread (a few values
+// spill on the general path): with 480-slot rows (16 warps, 128 registers) an
+// earlier form of the kernel took 8.16 ms, with 608 (20 warps, 96) 7.53, with
+// 736 7.20.
 constexpr int PUSH_THREADS = 736;           // pushing threads = slots per row
 constexpr int PUSH_WARPS = PUSH_THREADS / 32;
-constexpr int PUSH_BLOCK = PUSH_THREADS + 32;  // + one warp that streams the rows
 constexpr int PG = 1;           // guard cells around the tile
-constexpr int NSTAGE = 3;       // row ring stages (up to NSTAGE - 1 rows in flight)
-// Stages of the push's ring: the charge-only push (no current) has the
-// shared memory for one more.
-__host__ __device__ constexpr int push_stages(bool jd) { return jd ? NSTAGE : NSTAGE + 1; }
 constexpr int NJ = 12;          // zigzag node values of one cell
 constexpr int NR = 8;           // CIC node values of one cell
-constexpr int RQW = NJ + NR + 1;  // run-queue entry: 20 sums + box index of the cell (charge only: 8 + 1)
+// run-queue entry: the sums of a run (20, charge only 8), the box index of
+// its cell, one word of padding (the sums are stored in 8-byte pairs)
+__host__ __device__ constexpr int run_words(bool jd) { return (jd ? NJ + NR : NR) + 2; }
 constexpr int RQ_DRAIN = 8;     // drain the run queue at this many entries
-constexpr int RQCAP = RQ_DRAIN + 32;
+constexpr int RQ_ROUND = 16;    // lanes that put their run in the queue at a time
+constexpr int RQCAP = RQ_DRAIN + RQ_ROUND;
 constexpr int XQW = 8;          // general-path entry: slot, cell, 3 offsets, 3 velocities
-constexpr int XLCAP = 128;      // per-warp list of cross slots (emptied when nearly full)
-constexpr uint32_t ROW_BYTES = PUSH_THREADS * (16 + 3 * 4);
+constexpr int XLCAP = 96;       // per-warp list of cross slots (emptied when nearly full)
+constexpr int OLCAP = 64;       // per-warp list of out-of-place slots (a full batch is taken past 32)
+constexpr int RING = 3;         // rows of a warp's ring
+constexpr int ROW32 = 32 * (16 + 3 * 4);  // bytes of a row's 32 particles
+constexpr uint32_t NORUN = 0xFFFFFFFEu;  // no run open (cells have at most 31 bits)
 static_assert(PUSH_THREADS == EMSESG_FX_ROW_SLOTS, "row width of the thread-major layout");
-static_assert(ROW_BYTES % 16 == 0 && (PUSH_THREADS * 4) % 16 == 0, "bulk copies move whole 16-byte units");
 
 // Bodies of the FP32 form, in the order of cfg.body.  Box bodies (geotype
 // 0/1 with integer bounds): the absorption test and the per-surface-cell
@@ -124,9 +134,9 @@ struct FxPushArgs {
   const float* rvx;             // move-only step, those of a kept copy)
   const float* rvy;
   const float* rvz;
-  const int64_t* tile_start;    // [nspec][ntiles+1] sorted ranks (live particles)
-  const int64_t* tile_pad;      // [nspec][ntiles+1] slot offsets of the padded regions
   const int64_t* chunk_start;   // [nspec][ntiles+1] first CTA (row chunk) of each tile
+  const int4* chunks;           // [nspec][nchunk_max] the row chunks: tile, rows, first slot in the region
+  int64_t nchunk_max;
   int64_t off[EMSESG_ISPEC];    // region base per species
   int npbnd[EMSESG_ISPEC][3];
   float qmp[EMSESG_ISPEC], qfix[EMSESG_ISPEC];
@@ -138,7 +148,6 @@ struct FxPushArgs {
   FieldDesc fr, fj;
   Geo g;
   int64_t ntiles;
-  int chunk_rows;               // rows of a tile region per CTA
   int* nesc;                    // counter nesc(is), one int per species
   emsesg_counter* gc;           // influx / infhist of the body absorption
   unsigned long long* surf;     // [nspec][nsurf] absorbed - emitted counts
@@ -160,51 +169,58 @@ struct FxPushArgs {
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
-__device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
+// 16-byte copies global -> shared (both addresses 16-byte aligned), in groups.
+template <bool CA>
+__device__ __forceinline__ void cpa16(void* dst, const void* src) {
+  if (CA)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void mbar_fence_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cpa_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
-  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_u32(b)) : "memory");
+
+// ---------------------------------------------------------------- packed FP32
+// Two FP32 values in a 64-bit register pair: sm_100a's f32x2 instructions do
+// both in one issue slot, each rounded as the scalar instruction rounds it.
+// The pushing loop is bound by issue slots.  All arithmetic of the kick, the
+// move and the in-cell deposit is written with explicit roundings (these and
+// the __f*_rn intrinsics), so that every kernel that holds it gives the same
+// bits, however the compiler would fuse multiplies with adds.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
 }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
-  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(smem_u32(b)),
-               "r"(bytes)
-               : "memory");
+__device__ __forceinline__ f2 dup(float v) { return pk(v, v); }
+__device__ __forceinline__ void upk(f2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
+  f2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
-// Bounded wait: gives up after about one second.
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity) {
-  if (mbar_try_wait(b, parity)) return true;
-  const uint64_t t0 = global_ns();
-  for (uint32_t it = 0;; it++) {
-    if (mbar_try_wait(b, parity)) return true;
-    if ((it & 255u) == 255u && global_ns() - t0 > 1000000000ull) return false;
-  }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
-// 1-D bulk copy global -> shared, completing on an mbarrier (both addresses
-// 16-byte aligned, size a multiple of 16).
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
 }
+__device__ __forceinline__ f2 lerp2(f2 a, f2 b, f2 t) { return fma2(sub2(b, a), t, a); }
 
 // ---------------------------------------------------------------- moves
 // Per-axis move and outer boundary of psolve1.F90:366-606 on (cell, offset)
@@ -286,6 +302,18 @@ __host__ __device__ constexpr int rdi(int r) { return ((r & 3) == 1 || (r & 3) =
 __host__ __device__ constexpr int rdj(int r) { return (r & 3) >= 2 ? 1 : 0; }
 __host__ __device__ constexpr int rdk(int r) { return r < 4 ? 1 : 0; }
 
+// The tile's {Ex,Ey,Ez,Bx} nodes in shared memory have rows of 16 nodes for
+// the 11 of an 8-cell tile: neighbouring lanes hold neighbouring cells, and
+// with the next y row 16 nodes on, the 8 lanes of a 128-bit access that run
+// over a row's end (cells 0..7) fall on the 8 different 16-byte banks groups
+// again.  With rows of 11 a quarter of the gather's shared-memory passes were
+// bank conflicts.  {By,Bz} (64-bit accesses) keeps rows of 11.
+template <int B>
+struct FieldT {
+  static constexpr int W = B > 8 ? 16 : 8;  // row stride
+  static constexpr int N = W * B * B;
+};
+
 template <int B>
 struct BoxT {
   static constexpr int B2 = B * B;
@@ -325,6 +353,15 @@ template <int B>
 __device__ __forceinline__ int box_base(const int (&o)[3], int i, int j, int k) {
   int li = i - o[0], lj = j - o[1], lk = k - o[2];
   bool ok = (unsigned)li < (unsigned)(B - 1) && (unsigned)lj < (unsigned)(B - 1) && (unsigned)lk < (unsigned)(B - 1);
+  return ok ? (lk * B + lj) * B + li : -1;
+}
+
+// The same with the cell's index in the tile's {Ex,Ey,Ez,Bx} nodes.
+template <int B>
+__device__ __forceinline__ int box_base(const int (&o)[3], int i, int j, int k, int& fb) {
+  const int li = i - o[0], lj = j - o[1], lk = k - o[2];
+  const bool ok = (unsigned)li < (unsigned)(B - 1) && (unsigned)lj < (unsigned)(B - 1) && (unsigned)lk < (unsigned)(B - 1);
+  fb = (lk * B + lj) * FieldT<B>::W + li;
   return ok ? (lk * B + lj) * B + li : -1;
 }
 
@@ -420,66 +457,133 @@ __device__ __forceinline__ void gather8(const float4* f0, const void* f1v, int64
   b[0] = bx; b[1] = by; b[2] = bz;
 }
 
-// The same gather from the tile's shared-memory nodes (box index `base`,
-// compile-time strides).
-template <int B>
-__device__ __forceinline__ void gather8_smem(const float4* f0, const float2* f1, int base, const float (&w)[8],
-                                             float (&e)[3], float (&b)[3]) {
-  constexpr int SY = B, SZ = B * B;
-  constexpr int off[8] = {SZ, SZ + 1, SZ + 1 + SY, SZ + SY, 0, 1, 1 + SY, SY};
-  float ex = 0.f, ey = 0.f, ez = 0.f, bx = 0.f, by = 0.f, bz = 0.f;
+// E and B of a cell at the offsets (x, y, z): linear interpolations along x,
+// then y, then z, the six components in three pairs (Ex,Ey) (Ez,Bx) (By,Bz):
+// 42 packed operations (corner weights times values: 48 plus the weights).
+// n0(c) / n1(c): the node c (0..7: bit 0 x, bit 1 y, bit 2 z).
+struct EB { f2 exy, ezbx, byz; };
+template <class N0, class N1>
+__device__ __forceinline__ EB interp(float x, float y, float z, N0 n0, N1 n1) {
+  const f2 X = dup(x), Y = dup(y), Z = dup(z);
+  EB plane[2];
 #pragma unroll
-  for (int c = 0; c < 8; c++) {
-    const float4 p = f0[base + off[c]];
-    const float2 q = f1[base + off[c]];
-    ex += p.x * w[c];
-    ey += p.y * w[c];
-    ez += p.z * w[c];
-    bx += p.w * w[c];
-    by += q.x * w[c];
-    bz += q.y * w[c];
+  for (int k = 0; k < 2; k++) {
+    EB row[2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const ulonglong2 a0 = n0(4 * k + 2 * j), b0 = n0(4 * k + 2 * j + 1);
+      const f2 a1 = n1(4 * k + 2 * j), b1 = n1(4 * k + 2 * j + 1);
+      row[j] = EB{lerp2(a0.x, b0.x, X), lerp2(a0.y, b0.y, X), lerp2(a1, b1, X)};
+    }
+    plane[k] = EB{lerp2(row[0].exy, row[1].exy, Y), lerp2(row[0].ezbx, row[1].ezbx, Y),
+                  lerp2(row[0].byz, row[1].byz, Y)};
   }
-  e[0] = ex; e[1] = ey; e[2] = ez;
-  b[0] = bx; b[1] = by; b[2] = bz;
+  return EB{lerp2(plane[0].exy, plane[1].exy, Z), lerp2(plane[0].ezbx, plane[1].ezbx, Z),
+            lerp2(plane[0].byz, plane[1].byz, Z)};
 }
 
 // Trilinear gather of E and B at the particle (from the tile's shared nodes
 // when its cell lies in the box, gb >= 0, else from the global node field)
 // and the Buneman-Boris velocity update (psolve1.F90:186-272).  The shared
 // nodes hold the fields already multiplied by the species' qmp; the global
-// ones are multiplied here.
-template <int B>
-__device__ __forceinline__ void kick(const FxPushArgs& a, const float4* sf0, const float2* sf1, int gb, int ib, int jb,
-                                     int kb, const float4& ps, float qmp, float& vx, float& vy, float& vz) {
-  const float x1 = ps.x, y1 = ps.y, z1 = ps.z;
-  const float xy1 = x1 * y1, xz1 = x1 * z1, yz1 = y1 * z1, z2 = 1.0f - z1;
-  const float xz2 = x1 * z2, yz2 = y1 * z2;
-  float wv[8];
-  wv[2] = xy1 * z1; wv[1] = xz1 - wv[2]; wv[3] = yz1 - wv[2]; wv[0] = z1 - xz1 - wv[3];
-  wv[6] = xy1 * z2; wv[5] = xz2 - wv[6]; wv[7] = yz2 - wv[6]; wv[4] = z2 - xz2 - wv[7];
-  float fe[3], fb[3];
-  if (gb >= 0) {
-    gather8_smem<B>(sf0, sf1, gb, wv, fe, fb);
+// ones are multiplied here.  fb: the cell's index in the {Ex,Ey,Ez,Bx} nodes
+// (FieldT).  BOX: the cell is known to lie in the box.
+template <int B, bool BOX = false>
+__device__ __forceinline__ void kick(const FxPushArgs& a, const ulonglong2* sf0, const f2* sf1, int gb, int fb, int ib,
+                                     int jb, int kb, float x, float y, float z, float qmp, float& vx, float& vy,
+                                     float& vz) {
+  EB f;
+  if (BOX || gb >= 0) {
+    f = interp(
+        x, y, z,
+        [&](int c) { return sf0[fb + (c & 1) + ((c >> 1) & 1) * FieldT<B>::W + (c >> 2) * FieldT<B>::W * B]; },
+        [&](int c) { return sf1[gb + (c & 1) + ((c >> 1) & 1) * B + (c >> 2) * B * B]; });
   } else {
-    const int64_t sy = a.g.nx + 1, sz = (int64_t)(a.g.nx + 1) * (a.g.ny + 1);
-    gather8<false>(a.f0, a.f1, ib + sy * jb + sz * kb, sy, sz, wv, fe, fb);
+    const int64_t sy = a.g.nx + 1, sz = (int64_t)(a.g.nx + 1) * (a.g.ny + 1), n = ib + sy * jb + sz * kb;
+    f = interp(
+        x, y, z,
+        [&](int c) {
+          return __ldg(reinterpret_cast<const ulonglong2*>(a.f0) + n + (c & 1) + ((c >> 1) & 1) * sy + (c >> 2) * sz);
+        },
+        [&](int c) {
+          return __ldg(reinterpret_cast<const ulonglong2*>(a.f1) + n + (c & 1) + ((c >> 1) & 1) * sy + (c >> 2) * sz).x;
+        });
+    const f2 q = dup(qmp);
+    f.exy = mul2(f.exy, q);
+    f.ezbx = mul2(f.ezbx, q);
+    f.byz = mul2(f.byz, q);
+  }
+  float ex, ey, ez, bx, by, bz;
+  upk(f.exy, ex, ey);
+  upk(f.ezbx, ez, bx);
+  upk(f.byz, by, bz);
+  const float boris = __fdividef(2.0f, __fmaf_rn(bx, bx, __fmaf_rn(by, by, __fmaf_rn(bz, bz, 1.0f))));
+  vx = __fadd_rn(vx, ex);
+  vy = __fadd_rn(vy, ey);
+  vz = __fadd_rn(vz, ez);
+  const float vxt = __fmaf_rn(vy, bz, __fmaf_rn(-vz, by, vx));
+  const float vyt = __fmaf_rn(vz, bx, __fmaf_rn(-vx, bz, vy));
+  const float vzt = __fmaf_rn(vx, by, __fmaf_rn(-vy, bx, vz));
+  vx = __fmaf_rn(boris, __fmaf_rn(vyt, bz, -__fmul_rn(vzt, by)), vx);
+  vy = __fmaf_rn(boris, __fmaf_rn(vzt, bx, -__fmul_rn(vxt, bz)), vy);
+  vz = __fmaf_rn(boris, __fmaf_rn(vxt, by, -__fmul_rn(vyt, bx)), vz);
+  vx = __fadd_rn(vx, ex);
+  vy = __fadd_rn(vy, ey);
+  vz = __fadd_rn(vz, ez);
+}
+
+// The sums of a particle that stays in its cell, in pairs: with the current,
+// per component c of J the pairs 2c = (node value 1, 2) and 2c + 1 = (0, 3)
+// of jcomp's four, then the CIC values (r, r + 4) for r = 0..3.  Both zigzag
+// segments lie in the cell: relay point at the midpoint, equal segment
+// fluxes h = (a-b)/2/ustep, mid-points m -+ (a-b)/4; the sum of the two
+// bilinear weight sets is written with S = a+b, D = a-b.
+template <bool JD>
+__device__ __forceinline__ void cell_sums(float x, float y, float z, float sx, float sy, float sz, float hr,
+                                          f2 (&cv)[JD ? (NJ + NR) / 2 : NR / 2]) {
+  constexpr int RP = JD ? NJ / 2 : 0;  // first rho pair
+  if (JD) {
+    const f2 p = pk(x, y), s = pk(sx, sy);
+    const f2 Sxy = add2(s, p), Dxy = sub2(s, p);
+    const float Sz = __fadd_rn(sz, z), Dz = __fsub_rn(sz, z);
+    float Sx, Sy, Dx, Dy, hx, hy, Px, Py;
+    upk(Sxy, Sx, Sy);
+    upk(Dxy, Dx, Dy);
+    upk(mul2(Dxy, dup(hr)), hx, hy);
+    const float hz = __fmul_rn(Dz, hr);
+    upk(fma2(Dxy, dup(__fmul_rn(0.125f, Dz)), mul2(Sxy, dup(__fmul_rn(0.5f, Sz)))), Py, Px);
+    const float Pz = __fmaf_rn(__fmul_rn(0.125f, Dx), Dy, __fmul_rn(__fmul_rn(0.5f, Sx), Sy));
+    const float h3[3] = {hx, hy, hz}, P3[3] = {Px, Py, Pz};
+    const f2 ab[3] = {pk(Sy, Sz), pk(Sx, Sz), Sxy};  // S of the two other axes
+    const float ra[3] = {__fsub_rn(2.0f, Sy), __fsub_rn(2.0f, Sx), __fsub_rn(2.0f, Sx)};
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-      fe[d] *= qmp;
-      fb[d] *= qmp;
+    for (int c = 0; c < 3; c++) {
+      const f2 T = sub2(ab[c], dup(P3[c]));
+      float ta, tb;
+      upk(T, ta, tb);
+      cv[2 * c] = mul2(dup(h3[c]), T);
+      cv[2 * c + 1] = mul2(dup(h3[c]), pk(__fsub_rn(ra[c], tb), P3[c]));
     }
   }
-  const float eex = fe[0], eey = fe[1], eez = fe[2];
-  const float bbx = fb[0], bby = fb[1], bbz = fb[2];
-  const float boris = __fdividef(2.0f, 1.0f + bbx * bbx + bby * bby + bbz * bbz);
-  vx += eex; vy += eey; vz += eez;
-  const float vxt = vx + vy * bbz - vz * bby;
-  const float vyt = vy + vz * bbx - vx * bbz;
-  const float vzt = vz + vx * bby - vy * bbx;
-  vx += boris * (vyt * bbz - vzt * bby);
-  vy += boris * (vzt * bbx - vxt * bbz);
-  vz += boris * (vxt * bby - vyt * bbx);
-  vx += eex; vy += eey; vz += eez;
+  // CIC charge at the new position (charge.F90:152-210)
+  const f2 zz = pk(sz, __fsub_rn(1.0f, sz));
+  const f2 r2 = mul2(dup(__fmul_rn(sx, sy)), zz), XZ = mul2(dup(sx), zz);
+  const f2 r3 = sub2(mul2(dup(sy), zz), r2);
+  cv[RP + 2] = r2;
+  cv[RP + 1] = sub2(XZ, r2);
+  cv[RP + 3] = r3;
+  cv[RP + 0] = sub2(sub2(zz, XZ), r3);
+}
+
+// Box offset of sum i of that order.
+template <int B, bool JD>
+__host__ __device__ constexpr int sum_off(int i) {
+  constexpr int RO = JD ? NJ : 0;
+  if (JD && i < NJ) {
+    const int q = i & 3;
+    return BoxT<B>::joff((i & ~3) + (q == 0 ? 1 : q == 1 ? 2 : q == 2 ? 0 : 3));
+  }
+  return BoxT<B>::roff((i - RO) / 2 + ((i - RO) & 1) * 4);
 }
 
 // Empties a warp's run queue.  The queue's (entry, slot) items are dealt
@@ -491,7 +595,7 @@ template <int NC>
 __device__ __forceinline__ void drain_runs(unsigned long long* box, const int* slot_off, const float* q, int qn,
                                            float qfix, int lane) {
   static_assert(NC > 0 && NC <= 32, "an entry's sums fit one pass");
-  constexpr int QW = NC + 1;
+  constexpr int QW = NC + 2;
   __syncwarp();
   const int items = qn * NC;
   int e = lane / NC, sl = lane % NC;
@@ -509,6 +613,34 @@ __device__ __forceinline__ void drain_runs(unsigned long long* box, const int* s
     }
   }
   __syncwarp();
+}
+
+// The runs of the lanes in mk into the warp's queue, at most RQ_ROUND at a
+// time, emptied whenever RQ_DRAIN entries wait.
+template <int NC>
+__device__ __forceinline__ void queue_runs(unsigned long long* box, const int* slot_off, float* rq, int& rqn,
+                                           unsigned mk, bool mine, const f2 (&acc)[NC / 2], int base, float qfix,
+                                           int lane) {
+  constexpr int QW = NC + 2;
+  const unsigned lt = (1u << lane) - 1u;
+  int before = __popc(mk & lt);  // lanes to go before this one
+  int left = __popc(mk);
+  while (left > 0) {
+    if (mine && before >= 0 && before < RQ_ROUND) {
+      float* en = rq + (rqn + before) * QW;
+      f2* e2 = reinterpret_cast<f2*>(en);
+#pragma unroll
+      for (int q = 0; q < NC / 2; q++) e2[q] = acc[q];
+      en[NC] = __int_as_float(base);
+    }
+    rqn += min(left, RQ_ROUND);
+    before -= RQ_ROUND;
+    left -= RQ_ROUND;
+    if (rqn >= RQ_DRAIN) {
+      drain_runs<NC>(box, slot_off, rq, rqn, qfix, lane);
+      rqn = 0;
+    }
+  }
 }
 
 struct CrossCtx {
@@ -600,7 +732,7 @@ __device__ __forceinline__ int body_absorb(const CrossCtx& c, const int (&ib)[3]
 template <int B, bool DEP = true, bool CURV = true, bool JD = true>
 __device__ __forceinline__ int cross_one(const Geo& g, unsigned long long* box, const int (&o)[3], const Sink& sk,
                                          const CrossCtx& c, const float* en) {
-  const int loc = __float_as_int(en[0]);
+  const uint32_t loc = (uint32_t)__float_as_int(en[0]);
   const uint32_t cell = (uint32_t)__float_as_int(en[1]);
   const float bx = en[2], by = en[3], bz = en[4];
   float vx = en[5], vy = en[6], vz = en[7];
@@ -725,26 +857,101 @@ __device__ __forceinline__ int cross_one(const Geo& g, unsigned long long* box, 
 // gave them): each lane takes one and runs the general path.  Returns the
 // number of this lane's particles that escaped.
 template <int B, bool DEP, bool CURV, bool JD>
-__device__ __forceinline__ int cross_list(const FxPushArgs& a, int is, int64_t slot0, unsigned long long* box,
-                                          const int (&o)[3], const int* xl, int xn, int lane) {
+__device__ __forceinline__ int cross_list(const FxPushArgs& a, int is, unsigned long long* box,
+                                          const int (&o)[3], const uint32_t* xl, int xn, int lane) {
   __syncwarp();
   // the context comes from the kernel parameters here, so that the pushing
   // loop keeps none of it in registers
   const Geo& g = a.g;
   const Sink sk{a.acc_rho, a.acc_j, a.fr, a.fj, g.nx, g.ny, g.nz, a.status, a.diag};
-  const CrossCtx c{a.pos + slot0, a.vx + slot0, a.vy + slot0, a.vz + slot0, a.gustep, a.rustep, a.qfix[is],
+  const CrossCtx c{a.pos, a.vx, a.vy, a.vz, a.gustep, a.rustep, a.qfix[is],
                    {a.npbnd[is][0], a.npbnd[is][1], a.npbnd[is][2]}, &a.bd, a.gc,
-                   a.surf + (int64_t)is * a.bd.nsurf, is, slot0, a.ob.rec ? &a.ob : nullptr, a.status};
+                   a.surf + (int64_t)is * a.bd.nsurf, is, 0, a.ob.rec ? &a.ob : nullptr, a.status};
   int dead = 0;
   for (int e = lane; e < xn; e += 32) {
-    const int loc = xl[e];
-    const float4 ps = a.rpos[slot0 + loc];  // the position before the step
-    const float vx = c.gvx[loc], vy = c.gvy[loc], vz = c.gvz[loc];
-    const float en[XQW] = {__int_as_float(loc), ps.w, ps.x, ps.y, ps.z, vx, vy, vz};
+    const uint32_t m = xl[e];
+    const float4 ps = a.rpos[m];  // the position before the step
+    const float vx = c.gvx[m], vy = c.gvy[m], vz = c.gvz[m];
+    const float en[XQW] = {__int_as_float((int)m), ps.w, ps.x, ps.y, ps.z, vx, vy, vz};
     dead += cross_one<B, DEP, CURV, JD>(g, box, o, sk, c, en);
   }
   __syncwarp();
   return dead;
+}
+
+// An end point strictly inside its cell (a region next to a curved body
+// raises flo so that none is); one exactly on a face takes the general path
+// (it may lie on a body face: inclusive bounds).
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ bool in_cell(float sx, float sy, float sz, float flo) {
+  return min3(sx, sy, sz) > flo && max3(sx, sy, sz) < 1.0f;
+}
+
+// Out-of-place particles (in another cell than their column's run: they
+// changed cell since the sort, or lie outside the tile's box): each lane
+// takes one of the list's slots, e of en: kick and move; one that stays in
+// its cell adds its sums to the tile accumulator, the others join the warp's
+// cross list.  Taken 32 at a time: in the row loop a single such lane would
+// cost its warp the 20 sums' stores and most of a queue pass.
+template <int B, bool JD, bool PARTS>
+__device__ __forceinline__ int oop_list(const FxPushArgs& a, int is, unsigned long long* box,
+                                         const ulonglong2* sf0, const f2* sf1, const int (&o)[3], float flo,
+                                         const uint32_t* ol, int en, uint32_t* xl, int xqn, int lane) {
+  constexpr int NP = (JD ? NJ + NR : NR) / 2;
+  __syncwarp();
+  const Geo& g = a.g;
+  bool cross = false;
+  uint32_t m = 0;
+  if (lane < en) {
+    m = ol[lane];
+    const float4 ps = a.rpos[m];
+    float vx = a.rvx[m], vy = a.rvy[m], vz = a.rvz[m];
+    const uint32_t cell = (uint32_t)__float_as_int(ps.w);
+    int ib, jb, kb;
+    unpack(g, cell, ib, jb, kb);
+    int fb;
+    const int gb = box_base<B>(o, ib, jb, kb, fb);
+    if (PARTS && gb < 0 && kb + 1 > a.zready) {
+      // a part of a step whose eb arrives in z chunks: the node planes of this
+      // cell are not converted yet; left as it is for k_fx_deferred
+      atomicOr(a.defer + (m >> 5), 1u << (m & 31));
+    } else {
+      kick<B>(a, sf0, sf1, gb, fb, ib, jb, kb, ps.x, ps.y, ps.z, a.qmp[is], vx, vy, vz);
+      a.vx[m] = vx;
+      a.vy[m] = vy;
+      a.vz[m] = vz;
+      const float sx = __fmaf_rn(vx, a.gustep, ps.x), sy = __fmaf_rn(vy, a.gustep, ps.y),
+                  sz = __fmaf_rn(vz, a.gustep, ps.z);
+      if (gb >= 0 && in_cell(sx, sy, sz, flo)) {
+        a.pos[m] = make_float4(sx, sy, sz, ps.w);
+        f2 cv[NP];
+        cell_sums<JD>(ps.x, ps.y, ps.z, sx, sy, sz, 0.5f * a.rustep, cv);
+        const float qfix = a.qfix[is];
+#pragma unroll
+        for (int q = 0; q < NP; q++) {
+          float lo, hi;
+          upk(cv[q], lo, hi);
+          box_add(&box[gb + sum_off<B, JD>(2 * q)], (unsigned long long)to_fix(lo, qfix));
+          box_add(&box[gb + sum_off<B, JD>(2 * q + 1)], (unsigned long long)to_fix(hi, qfix));
+        }
+      } else {
+        cross = true;
+      }
+    }
+  }
+  const unsigned xm = __ballot_sync(0xffffffffu, cross);
+  if (cross) xl[xqn + __popc(xm & ((1u << lane) - 1u))] = m;
+  __syncwarp();
+  return xqn + __popc(xm);
 }
 
 // DEP = false: the move only (positions, velocities, boundary rules; no
@@ -757,85 +964,71 @@ __device__ __forceinline__ int cross_list(const FxPushArgs& a, int is, int64_t s
 // the charge only -- runs of 8 CIC sums, an accumulator of rho alone, no
 // zigzag current.
 template <int T, bool DEP = true, bool CURV = false, bool JD = true, bool PARTS = false>
-__global__ void __launch_bounds__(PUSH_BLOCK, 1) k_fx_push(FxPushArgs a) {
+__global__ void __launch_bounds__(PUSH_THREADS, 1) k_fx_push(const __grid_constant__ FxPushArgs a) {
   constexpr int B = T + 2 * PG + 1;  // box and field tile edge (nodes)
   constexpr int NC = JD ? NJ + NR : NR;  // sums of a run: zigzag J and CIC rho, or rho alone
-  constexpr int RO = JD ? NJ : 0;        // first rho sum
-  constexpr int QW = NC + 1;             // run-queue entry: the sums and the cell's box index
+  constexpr int NP = NC / 2;             // in pairs
+  constexpr int QW = run_words(JD);      // run-queue entry
   constexpr int NACC = (JD ? 4 : 1) * B * B * B;  // accumulator entries (rho, then Jx, Jy, Jz)
-  constexpr int NBOX = (NACC + 1) & ~1;           // their 8-byte words, padded so that the ring after them
-                                                  // starts on a 16-byte boundary (bulk copies, float4)
+  constexpr int NBOX = (NACC + 1) & ~1;  // their 8-byte words, padded: the field nodes after them are float4
   constexpr int NF = B * B * B;
-  constexpr int NS = push_stages(JD);  // row ring stages
-  static_assert((NBOX * 8) % 16 == 0 && (NBOX * 8 + NS * ROW_BYTES) % 16 == 0,
-                "the row ring and the field tile start on 16-byte boundaries");
+  static_assert((NBOX * 8) % 16 == 0, "the field tile starts on a 16-byte boundary");
   extern __shared__ __align__(128) unsigned long long smem[];
-  __shared__ __align__(8) uint64_t full_bar[NS];
-  __shared__ __align__(8) uint64_t empty_bar[NS];
   __shared__ int slot_off[NC];
-  __shared__ int rows_seen;
   const Geo& g = a.g;
   const int is = blockIdx.y;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   const unsigned lt = (1u << lane) - 1u;
 
-  // this CTA's chunk: tile t, rows r0 .. r0 + L - 1 of its region (a tile of
-  // more than CHUNK_ROWS rows is pushed by several CTAs, which add their
-  // sums into the same global arrays)
-  const int64_t* ts = a.tile_start + (int64_t)is * (a.ntiles + 1);
+  // this CTA's row chunk (a tile of more than chunk_rows rows is pushed by
+  // several CTAs, which add their sums into the same global arrays), from the
+  // table the sort leaves: one load instead of a binary search over the tiles'
+  // first chunks, a chain of dependent loads in front of everything else
   const int64_t* cs = a.chunk_start + (int64_t)is * (a.ntiles + 1);
-  const int64_t t_end = a.t_n > 0 ? a.t_lo + a.t_n : a.ntiles;
-  const int64_t b = cs[a.t_lo] + blockIdx.x;
-  if (b >= cs[t_end]) return;
-  int64_t tlo = a.t_lo, thi = t_end;  // the last tile with cs[t] <= b
-  while (thi - tlo > 1) {
-    const int64_t mid = (tlo + thi) >> 1;
-    if (cs[mid] <= b) tlo = mid;
-    else thi = mid;
-  }
-  const int t = (int)tlo;
-  const int64_t n = ts[t + 1] - ts[t];
-  if (n <= 0) return;
-  const int r0 = (int)(b - cs[t]) * a.chunk_rows;
-  const int L = min((int)((n + PUSH_THREADS - 1) / PUSH_THREADS) - r0, a.chunk_rows);
-  if (L <= 0) return;
-  const int64_t slot0 = a.off[is] + a.tile_pad[(int64_t)is * (a.ntiles + 1) + t] + (int64_t)r0 * PUSH_THREADS;
+  const int64_t b = (a.t_lo > 0 ? cs[a.t_lo] : 0) + blockIdx.x;
+  const int4 chunk = b < a.nchunk_max ? __ldg(a.chunks + (int64_t)is * a.nchunk_max + b) : make_int4(0, 0, 0, 0);
+  if (b >= cs[a.t_n > 0 ? a.t_lo + a.t_n : a.ntiles]) return;
+  const int t = chunk.x, L = chunk.y;
+  const int64_t slot0 = a.off[is] + (uint32_t)chunk.z;
 
   int tx = t % g.nt[0], ty = (t / g.nt[0]) % g.nt[1], tz = t / (g.nt[0] * g.nt[1]);
   const int o[3] = {tx * g.t[0] - PG, ty * g.t[1] - PG, tz * g.t[2] - PG};
   unsigned long long* box = smem;
-  float4* stpos = reinterpret_cast<float4*>(smem + NBOX);
-  float* stvx = reinterpret_cast<float*>(stpos + NS * PUSH_THREADS);
-  float* stvy = stvx + NS * PUSH_THREADS;
-  float* stvz = stvy + NS * PUSH_THREADS;
-  float4* sf0 = reinterpret_cast<float4*>(stvz + NS * PUSH_THREADS);
-  float2* sf1 = reinterpret_cast<float2*>(sf0 + NF);
-  float* rq = reinterpret_cast<float*>(sf1 + NF) + warp * RQCAP * QW;
-  int* xl = reinterpret_cast<int*>(reinterpret_cast<float*>(sf1 + NF) + PUSH_WARPS * RQCAP * QW) + warp * XLCAP;
+  float4* sf0 = reinterpret_cast<float4*>(smem + NBOX);
+  float2* sf1 = reinterpret_cast<float2*>(sf0 + FieldT<B>::N);
+  float* rq = reinterpret_cast<float*>(sf1 + (NF + 1) / 2 * 2) + warp * RQCAP * QW;
+  uint32_t* xl = reinterpret_cast<uint32_t*>(reinterpret_cast<float*>(sf1 + (NF + 1) / 2 * 2) + PUSH_WARPS * RQCAP * QW) +
+                 warp * (XLCAP + OLCAP);
+  uint32_t* ol = xl + XLCAP;
+  constexpr int ring_off = NBOX * 8 + FieldT<B>::N * 16 + (NF + 1) / 2 * 16 +
+                           PUSH_WARPS * (RQCAP * QW * 4 + (XLCAP + OLCAP) * 4);
+  static_assert(ring_off % 16 == 0 && ROW32 % 16 == 0, "16-byte copies");
 
-  float4* gpos = a.pos + slot0;
-  float* gvx = a.vx + slot0;
-  float* gvy = a.vy + slot0;
-  float* gvz = a.vz + slot0;
-  const float4* rgpos = a.rpos + slot0;
-  const float* rgvx = a.rvx + slot0;
-  const float* rgvy = a.rvy + slot0;
-  const float* rgvz = a.rvz + slot0;
+  // slots are addressed by 32-bit indices from the arrays in the kernel's
+  // parameters: eight 64-bit bases would take 16 of the 80 registers
+  const uint32_t sl0 = (uint32_t)slot0 + tid;
 
-  if (tid == 0) {
-    for (int s = 0; s < NS; s++) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], PUSH_WARPS);
+  char* const ring = reinterpret_cast<char*>(smem) + ring_off + warp * (RING * ROW32);
+  // lane 8 q + c of the first 24 copies the c-th 16 bytes of the q-th velocity
+  const float* vsrc = (lane < 8 ? a.rvx : lane < 16 ? a.rvy : a.rvz) + (sl0 - lane + 4 * (lane & 7));
+  auto fetch = [&](int row, uint32_t slot, char* to) {
+    if (row < L) {
+      cpa16<false>(to + lane * 16, a.rpos + slot);
+      if (lane < 24) cpa16<false>(to + 512 + lane * 16, vsrc);
     }
-    mbar_fence_init();
-  }
-  if (tid < NC) slot_off[tid] = tid < RO ? BoxT<B>::joff(tid) : BoxT<B>::roff(tid - RO);
+    vsrc += PUSH_THREADS;
+    cpa_commit();
+  };
+  fetch(0, sl0, ring);
+  fetch(1, sl0 + PUSH_THREADS, ring + ROW32);
+
+  if (tid < NC) slot_off[tid] = sum_off<B, JD>(tid);
   if (DEP)
-    for (int e = tid; e < NBOX; e += PUSH_BLOCK) box[e] = 0ull;
+    for (int e = tid; e < NBOX; e += PUSH_THREADS) box[e] = 0ull;
   const int64_t sy = g.nx + 1, sz = (int64_t)(g.nx + 1) * (g.ny + 1);
   const float sq = a.qmp[is];  // the tile's fields times the species' qmp
-  for (int e = tid; e < NF; e += PUSH_BLOCK) {
+  for (int e = tid; e < NF; e += PUSH_THREADS) {
     int li = e % B, lj = (e / B) % B, lk = e / (B * B);
     int gi = o[0] + li, gj = o[1] + lj, gk = o[2] + lk;
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p;
@@ -844,36 +1037,15 @@ __global__ void __launch_bounds__(PUSH_BLOCK, 1) k_fx_push(FxPushArgs a) {
       p = __ldg(&a.f0[gn]);
       q = __ldg(&a.f1[gn]);
     }
-    sf0[e] = make_float4(p.x * sq, p.y * sq, p.z * sq, p.w * sq);
+    sf0[(lk * B + lj) * FieldT<B>::W + li] = make_float4(p.x * sq, p.y * sq, p.z * sq, p.w * sq);
     sf1[e] = make_float2(q.x * sq, q.y * sq);
   }
   __syncthreads();
 
-  int issued = 0;  // rows issued (producer lane 0)
-  if (warp == PUSH_WARPS) {
-    // Row producer: row r goes to stage r % NS once every pushing warp
-    // released the row that used that stage before.
-    if (lane == 0) {
-      for (int r = 0; r < L; r++) {
-        const int s = r % NS;
-        if (r >= NS && !mbar_wait(&empty_bar[s], (uint32_t)((r / NS - 1) & 1))) {
-          report_bad(a.status, a.diag, SITE_FX_PUSH, -4, t);
-          break;
-        }
-        mbar_expect_tx(&full_bar[s], ROW_BYTES);
-        const int64_t ro = (int64_t)r * PUSH_THREADS;
-        bulk_g2s(stpos + s * PUSH_THREADS, rgpos + ro, PUSH_THREADS * 16, &full_bar[s]);
-        bulk_g2s(stvx + s * PUSH_THREADS, rgvx + ro, PUSH_THREADS * 4, &full_bar[s]);
-        bulk_g2s(stvy + s * PUSH_THREADS, rgvy + ro, PUSH_THREADS * 4, &full_bar[s]);
-        bulk_g2s(stvz + s * PUSH_THREADS, rgvz + ro, PUSH_THREADS * 4, &full_bar[s]);
-        issued = r + 1;
-      }
-    }
-    __syncwarp();
-  } else {
-
-  const float qmp = a.qmp[is], qfix = a.qfix[is];
+  const float qfix = a.qfix[is];
   const float gustep = a.gustep, hr = 0.5f * a.rustep;
+  const ulonglong2* f0s = reinterpret_cast<const ulonglong2*>(sf0);
+  const f2* f1s = reinterpret_cast<const f2*>(sf1);
   // A particle can end inside a body without leaving its cell (entering a
   // cylinder or a sphere, or starting inside any body, where the reference's
   // end-point test absorbs it): in a tile region whose box touches a body's
@@ -889,229 +1061,162 @@ __global__ void __launch_bounds__(PUSH_BLOCK, 1) k_fx_push(FxPushArgs a) {
       if (hit) flo = 2.0f;
     }
 
-  float acc[NC];
+  f2 acc[NP];
 #pragma unroll
-  for (int s = 0; s < NC; s++) acc[s] = 0.f;
-  uint32_t runcell = DEAD;
-  int runbase = -1;
+  for (int s = 0; s < NP; s++) acc[s] = 0ull;
+  uint32_t runcell = NORUN;
+  int runbase = -1, runfb = 0;
   int nesc = 0;
-  int rqn = 0, xqn = 0;  // warp-uniform queue lengths
-  bool failed = false;
-  int seen = 0;  // rows observed complete (thread 0)
-  // Row r is pushed while row r+1 is already in shared memory: the cell of
-  // the thread's next particle decides whether a change of cell starts a new
-  // run or is a single particle out of place (one that changed cell since
-  // the sort), which then takes the cross path and leaves the run intact.
-  bool okme = false;
-  if (L > 0) {
-    okme = mbar_wait(&full_bar[0], 0u);
-    if (!__any_sync(0xffffffffu, okme)) failed = true;
-    for (int k = 0; !okme && k < 1024; k++) okme = mbar_try_wait(&full_bar[0], 0u);
-    if (tid == 0 && okme) seen = 1;
-  }
+  int rqn = 0, xqn = 0, oqn = 0;  // warp-uniform queue lengths
 
+  // Row r is read while row r + 1 is in shared memory and r + 2 under way
+  // (cp.async into the warp's own ring: the warps share no barrier and no
+  // registers hold rows in flight).  The cell of the thread's next particle
+  // decides whether a change of cell starts a new run or is a single particle
+  // out of place (one that changed cell since the sort: the next one is back in
+  // the run's cell), which goes on the out-of-place list and leaves the run
+  // intact.
+  uint32_t sl = sl0;  // this thread's slot of row r
+  int at = 0, at2 = 2 * ROW32;  // the stages of rows r and r + 2
   int r = 0;
-  for (;;) {
-  // the stage of row r and the parity of its use, kept as running counters
-  int s = r % NS;
-  uint32_t ph = (uint32_t)((r / NS) & 1);
-  for (; r < L && !failed; r++) {
-    const int s1 = s + 1 == NS ? 0 : s + 1;
-    const uint32_t par1 = s1 == 0 ? ph ^ 1u : ph;
-    uint32_t nextcell = DEAD;
-    bool oknext = false;
-    if (r + 1 < L) {
-      oknext = mbar_wait(&full_bar[s1], par1);
-      if (!__any_sync(0xffffffffu, oknext)) {
-        failed = true;
-        break;
-      }
-      for (int k = 0; !oknext && k < 1024; k++) oknext = mbar_try_wait(&full_bar[s1], par1);
-      if (tid == 0 && oknext) seen = r + 2;
-      if (oknext) nextcell = (uint32_t)__float_as_int(stpos[s1 * PUSH_THREADS + tid].w);
-    }
-    const float4 ps = stpos[s * PUSH_THREADS + tid];
-    float vx = stvx[s * PUSH_THREADS + tid];
-    float vy = stvy[s * PUSH_THREADS + tid];
-    float vz = stvz[s * PUSH_THREADS + tid];
+  while (r < L) {
+  for (; r < L; r++) {
+    __syncwarp();  // every lane is through with the row that leaves the ring
+    fetch(r + 2, sl + 2 * PUSH_THREADS, ring + at2);
+    cpa_wait<1>();
     __syncwarp();
-    if (lane == 0) mbar_arrive(&empty_bar[s]);
-
+    const char* row = ring + at;
+    const float4 ps = *reinterpret_cast<const float4*>(row + lane * 16);
+    const float* rv = reinterpret_cast<const float*>(row + 512) + lane;
+    float vx = rv[0], vy = rv[32], vz = rv[64];
+    at2 = at;  // row r + 3 takes this stage
+    at = at + ROW32 == RING * ROW32 ? 0 : at + ROW32;
+    uint32_t nextcell = DEAD;
+    if (r + 1 < L) nextcell = *reinterpret_cast<const uint32_t*>(ring + at + lane * 16 + 12);
     const uint32_t cell = (uint32_t)__float_as_int(ps.w);
-    bool act = cell != DEAD && okme;
-    okme = oknext;
-    int ib = 0, jb = 0, kb = 0;
-    if (act) {
-      unpack(g, cell, ib, jb, kb);
-      if (ib >= g.nx || jb >= g.ny || kb >= g.nz) {
-        report_bad(a.status, a.diag, SITE_FX_PUSH, slot0 + (int64_t)r * PUSH_THREADS + tid, (long long)cell);
-        act = false;
-      }
-    }
-    // ---- a new cell ends the thread's run (its sums go to the run queue)
-    // when the next particle is in that cell too, or when there is no run
-    const bool newrun = DEP && act && cell != runcell && (runbase < 0 || nextcell == cell || nextcell == DEAD);
+    bool cross = false;
     if (DEP) {
-      const bool evict = newrun && runbase >= 0;
+      // ---- a particle in another cell than the thread's run: it ends the
+      // run (whose sums go to the run queue) and starts its own, or it is out
+      // of place
+      bool in = cell == runcell, newrun = false, oop = false;
+      int base = runbase, fb = runfb;
+      if (!in && cell != DEAD) {
+        int ib, jb, kb;
+        unpack(g, cell, ib, jb, kb);
+        if (ib < g.nx && jb < g.ny && kb < g.nz) {
+          base = box_base<B>(o, ib, jb, kb, fb);
+          newrun = base >= 0 && (runcell == NORUN || nextcell != runcell);
+          oop = !newrun;
+        } else {
+          report_bad(a.status, a.diag, SITE_FX_PUSH, (int64_t)sl, (long long)cell);
+        }
+      }
+      const bool evict = newrun && runcell != NORUN;
       const unsigned mk = __ballot_sync(0xffffffffu, evict);
-      if (mk) {
-        if (evict) {
-          float* en = rq + (rqn + __popc(mk & lt)) * QW;
+      if (mk) queue_runs<NC>(box, slot_off, rq, rqn, mk, evict, acc, runbase, qfix, lane);
+      const unsigned om = __ballot_sync(0xffffffffu, oop);
+      if (oop) ol[oqn + __popc(om & lt)] = sl;
+      oqn += __popc(om);
+      // a new run starts from zero: folded into this particle's accumulate
+      const f2 keep = dup(newrun ? 0.f : 1.f);
+      if (newrun) {
+        runcell = cell;
+        runbase = base;
+        runfb = fb;
+        in = true;
+      }
+      // ---- gather + Buneman-Boris (psolve1.F90:186-272), the move and, in
+      // the cell, the sums
+      if (in) {
+        kick<B, true>(a, f0s, f1s, runbase, runfb, 0, 0, 0, ps.x, ps.y, ps.z, 0.f, vx, vy, vz);
+        const float sx = __fmaf_rn(vx, gustep, ps.x), sy = __fmaf_rn(vy, gustep, ps.y),
+                    sz = __fmaf_rn(vz, gustep, ps.z);
+        // the new velocity of every particle (a cell-crossing one keeps its
+        // old position until the general path writes the whole record)
+        a.vx[sl] = vx;
+        a.vy[sl] = vy;
+        a.vz[sl] = vz;
+        if (in_cell(sx, sy, sz, flo)) {
+          a.pos[sl] = make_float4(sx, sy, sz, ps.w);
+          f2 cv[NP];
+          cell_sums<JD>(ps.x, ps.y, ps.z, sx, sy, sz, hr, cv);
 #pragma unroll
-          for (int q = 0; q < NC; q++) en[q] = acc[q];
-          en[NC] = __int_as_float(runbase);
+          for (int q = 0; q < NP; q++) acc[q] = fma2(acc[q], keep, cv[q]);
+        } else {
+          cross = true;
+          if (newrun) runcell = NORUN;
         }
-        rqn += __popc(mk);
-        if (rqn >= RQ_DRAIN) {
-          drain_runs<NC>(box, slot_off, rq, rqn, qfix, lane);
-          rqn = 0;
-        }
       }
-    }
-    // a new run starts from zero: folded into this particle's accumulate
-    // below, or (rarely: the particle itself leaves the run's cell) cleared
-    const float keep = newrun ? 0.f : 1.f;
-    if (newrun) {
-      runcell = cell;
-      runbase = box_base<B>(o, ib, jb, kb);
-    }
-
-    // ---- gather + Buneman-Boris (psolve1.F90:186-272)
-    bool simple = false, oop = false, defer = false;
-    int gb = -1;
-    float sx = 0.f, syy = 0.f, szz = 0.f;
-    if (act) {
-      gb = cell == runcell ? runbase : box_base<B>(o, ib, jb, kb);
-      // a part of a step whose eb arrives in z chunks: a cell outside the box
-      // (a particle that crossed a periodic face or left the box since the
-      // sort) whose node planes are not converted yet is left as it is for
-      // k_fx_deferred
-      defer = PARTS && gb < 0 && kb + 1 > a.zready;
-      if (defer) {
-        const int64_t m = slot0 + (int64_t)r * PUSH_THREADS + tid;
-        atomicOr(a.defer + (m >> 5), 1u << (m & 31));
+    } else if (cell != DEAD) {
+      // a move-only step
+      int ib, jb, kb;
+      unpack(g, cell, ib, jb, kb);
+      if (ib < g.nx && jb < g.ny && kb < g.nz) {
+        int fb;
+        const int gb = box_base<B>(o, ib, jb, kb, fb);
+        kick<B>(a, f0s, f1s, gb, fb, ib, jb, kb, ps.x, ps.y, ps.z, a.qmp[is], vx, vy, vz);
+        const float sx = __fmaf_rn(vx, gustep, ps.x), sy = __fmaf_rn(vy, gustep, ps.y),
+                    sz = __fmaf_rn(vz, gustep, ps.z);
+        cross = !in_cell(sx, sy, sz, flo);
+        if (!cross) a.pos[sl] = make_float4(sx, sy, sz, ps.w);
       } else {
-        kick<B>(a, sf0, sf1, gb, ib, jb, kb, ps, qmp, vx, vy, vz);
-        sx = ps.x + vx * gustep;
-        syy = ps.y + vy * gustep;
-        szz = ps.z + vz * gustep;
-        // an end point exactly on a cell face takes the general path (it may
-        // lie on a body face: inclusive bounds)
-        const bool incell = sx > flo && sx < 1.0f && syy > 0.f && syy < 1.0f && szz > 0.f && szz < 1.0f;
-        simple = incell && (!DEP || (cell == runcell && runbase >= 0));
-        // a particle that stays in its cell but is out of place in the thread's
-        // run (it changed cell since the sort): its 20 sums go to the run queue
-        oop = DEP && incell && !simple && gb >= 0;
+        report_bad(a.status, a.diag, SITE_FX_PUSH, (int64_t)sl, (long long)cell);
+        a.pos[sl] = ps;
       }
-    }
-    const unsigned om = DEP ? __ballot_sync(0xffffffffu, oop) : 0u;
-    float* oen = oop ? rq + (rqn + __popc(om & lt)) * QW : nullptr;
-    if (DEP && (simple || oop)) {
-      // both zigzag segments in the same cell: relay point at the midpoint,
-      // equal segment fluxes h = (a-b)/2/ustep, mid-points m -+ (a-b)/4; the
-      // sum of the two bilinear weight sets is written with S = a+b, D = a-b
-      float cv[NC];
-      if (JD) {
-        const float Sx = sx + ps.x, Sy = syy + ps.y, Sz = szz + ps.z;
-        const float Dx = sx - ps.x, Dy = syy - ps.y, Dz = szz - ps.z;
-        const float hx = Dx * hr, hy = Dy * hr, hz = Dz * hr;
-        float P;
-        P = 0.5f * Sy * Sz + 0.125f * Dy * Dz;
-        cv[3] = hx * P; cv[1] = hx * (Sy - P); cv[2] = hx * (Sz - P); cv[0] = hx * (2.0f - Sy - Sz + P);
-        P = 0.5f * Sx * Sz + 0.125f * Dx * Dz;
-        cv[7] = hy * P; cv[5] = hy * (Sx - P); cv[6] = hy * (Sz - P); cv[4] = hy * (2.0f - Sx - Sz + P);
-        P = 0.5f * Sx * Sy + 0.125f * Dx * Dy;
-        cv[11 % NC] = hz * P; cv[9 % NC] = hz * (Sx - P); cv[10 % NC] = hz * (Sy - P);
-        cv[8 % NC] = hz * (2.0f - Sx - Sy + P);
-      }
-      // CIC charge at the new position (charge.F90:152-210)
-      const float XY = sx * syy, XZ = sx * szz, YZ = syy * szz, Z2 = 1.0f - szz, XZ2 = sx * Z2, YZ2 = syy * Z2;
-      const float r2 = XY * szz, r6 = XY * Z2;
-      const float r3 = YZ - r2, r7 = YZ2 - r6;
-      cv[RO + 2] = r2; cv[RO + 1] = XZ - r2; cv[RO + 3] = r3; cv[RO + 0] = szz - XZ - r3;
-      cv[RO + 6] = r6; cv[RO + 5] = XZ2 - r6; cv[RO + 7] = r7; cv[RO + 4] = Z2 - XZ2 - r7;
-      if (oop) {
-#pragma unroll
-        for (int q = 0; q < NC; q++) oen[q] = cv[q];
-        oen[NC] = __int_as_float(gb);
-      } else {
-#pragma unroll
-        for (int q = 0; q < NC; q++) acc[q] = fmaf(acc[q], keep, cv[q]);
-      }
-    }
-    if (newrun && !simple) {
-#pragma unroll
-      for (int q = 0; q < NC; q++) acc[q] = 0.f;
-    }
-    // the new velocity of every particle (a cell-crossing one keeps its old
-    // position until the general path writes the whole record)
-    if (act && !defer) {
-      const int m = r * PUSH_THREADS + tid;
-      if (simple || oop) gpos[m] = make_float4(sx, syy, szz, ps.w);
-      gvx[m] = vx;
-      gvy[m] = vy;
-      gvz[m] = vz;
-    } else if (!DEP) {
-      // a move-only step may write into other arrays than it reads: empty
-      // and dead slots are carried over
-      const int m = r * PUSH_THREADS + tid;
-      gpos[m] = ps;
-      gvx[m] = vx;
-      gvy[m] = vy;
-      gvz[m] = vz;
-    }
-    if (om) {
-      rqn += __popc(om);
-      if (rqn >= RQ_DRAIN) {
-        drain_runs<NC>(box, slot_off, rq, rqn, qfix, lane);
-        rqn = 0;
-      }
+      a.vx[sl] = vx;
+      a.vy[sl] = vy;
+      a.vz[sl] = vz;
+    } else {
+      // it may write into other arrays than it reads: empty and dead slots
+      // are carried over
+      a.pos[sl] = ps;
+      a.vx[sl] = vx;
+      a.vy[sl] = vy;
+      a.vz[sl] = vz;
     }
     // ---- cell-crossing particles: the warp's cross list (their positions
     // stay as they were; the general path after the row loop moves them)
-    const bool cross = act && !simple && !oop && !defer;
     const unsigned xm = __ballot_sync(0xffffffffu, cross);
-    if (xm) {
-      if (cross) xl[xqn + __popc(xm & lt)] = r * PUSH_THREADS + tid;
-      xqn += __popc(xm);
-      if (xqn > XLCAP - 32) {  // full: empty it, then go on with the next row
-        r++;
-        break;
-      }
+    if (cross) xl[xqn + __popc(xm & lt)] = sl;
+    xqn += __popc(xm);
+    sl += PUSH_THREADS;
+    if (xqn > XLCAP - 32 || oqn > OLCAP - 32) {  // take full batches, then go on with the next row
+      r++;
+      break;
     }
-    s = s1;
-    ph = par1;
   }
-  if (xqn) {
-    nesc += cross_list<B, DEP, CURV, JD>(a, is, slot0, box, o, xl, xqn, lane);
-    xqn = 0;
-  }
-  if (r >= L || failed) break;
-  }
-  if (failed) report_bad(a.status, a.diag, SITE_FX_PUSH, -3, t);
-  // the last run of every thread, and what is left in the queues
+  // the lists: whole batches of 32 while rows are left, everything at the end
+  const bool last = r >= L;
   if (DEP) {
-    const bool has = runbase >= 0;
-    const unsigned mk = __ballot_sync(0xffffffffu, has);
-    if (has) {
-      float* en = rq + (rqn + __popc(mk & lt)) * QW;
-#pragma unroll
-      for (int q = 0; q < NC; q++) en[q] = acc[q];
-      en[NC] = __int_as_float(runbase);
+    while (oqn >= 32 || (last && oqn > 0)) {
+      const int k = min(oqn, 32);
+      oqn -= k;
+      if (xqn > XLCAP - 32) {
+        xqn -= 32;
+        nesc += cross_list<B, DEP, CURV, JD>(a, is, box, o, xl + xqn, 32, lane);
+      }
+      xqn = oop_list<B, JD, PARTS>(a, is, box, f0s, f1s, o, flo, ol + oqn, k, xl, xqn, lane);
     }
-    rqn += __popc(mk);
+  }
+  while (xqn > XLCAP - 32 || (last && xqn > 0)) {
+    const int k = min(xqn, 32);
+    xqn -= k;
+    nesc += cross_list<B, DEP, CURV, JD>(a, is, box, o, xl + xqn, k, lane);
+  }
+  }
+  // the last run of every thread, and what is left in the queue
+  if (DEP) {
+    const bool has = runcell != NORUN;
+    const unsigned mk = __ballot_sync(0xffffffffu, has);
+    if (mk) queue_runs<NC>(box, slot_off, rq, rqn, mk, has, acc, runbase, qfix, lane);
     if (rqn) drain_runs<NC>(box, slot_off, rq, rqn, qfix, lane);
   }
   if (nesc) atomicAdd(&a.nesc[is], nesc);
-  if (tid == 0) rows_seen = seen;
-  }  // pushing warps
   __syncthreads();
-  // copies still in flight after a failed wait complete before the CTA exits
-  if (warp == PUSH_WARPS && lane == 0)
-    for (int r = rows_seen; r < issued; r++) (void)mbar_wait(&full_bar[r % NS], (uint32_t)((r / NS) & 1));
   // add the tile accumulator into the global int64 arrays
   if (DEP) {
-    for (int e = tid; e < NACC; e += PUSH_BLOCK) {
+    for (int e = tid; e < NACC; e += PUSH_THREADS) {
       unsigned long long v = box[e];
       if (v == 0ull) continue;
       int li = e % B, lj = (e / B) % B, lk = (e / (B * B)) % B, comp = e / (B * B * B);
@@ -1133,22 +1238,30 @@ __global__ void __launch_bounds__(PUSH_BLOCK, 1) k_fx_push(FxPushArgs a) {
   }
 }
 
+// The entries of tile t's row chunks (FxPushArgs::chunks) from its first one.
+__device__ __forceinline__ void put_chunks(int4* out, int64_t first, int64_t t, int64_t rows, int64_t slot,
+                                           int chunk_rows) {
+  for (int64_t r = 0; r < rows; r += chunk_rows)
+    out[first++] = make_int4((int)t, (int)min((int64_t)chunk_rows, rows - r), (int)(uint32_t)(slot + r * PUSH_THREADS), 0);
+}
+
 // The row chunks of every tile region: cs[t] = first chunk of tile t,
-// cs[ntiles] = the number of chunks (one block of 1024 threads per species).
-__global__ void __launch_bounds__(1024) k_push_chunks(const int64_t* __restrict__ tile_start, int64_t ntiles,
-                                                      int64_t* chunk_start, int chunk_rows) {
+// cs[ntiles] = the number of chunks (one block of 1024 threads per species),
+// and their entries.
+__global__ void __launch_bounds__(1024) k_push_chunks(const int64_t* __restrict__ tile_start,
+                                                      const int64_t* __restrict__ tile_pad, int64_t ntiles,
+                                                      int64_t* chunk_start, int4* chunks, int64_t nchunk_max,
+                                                      int chunk_rows) {
   __shared__ int64_t pa[1024];
   const int64_t* ts = tile_start + (int64_t)blockIdx.x * (ntiles + 1);
+  const int64_t* tp = tile_pad + (int64_t)blockIdx.x * (ntiles + 1);
   int64_t* cs = chunk_start + (int64_t)blockIdx.x * (ntiles + 1);
   const int tid = threadIdx.x;
   const int64_t per = (ntiles + 1023) / 1024;
   const int64_t t0 = tid * per, t1 = min(ntiles, t0 + per);
-  auto chunks = [&](int64_t t) {
-    const int64_t rows = (ts[t + 1] - ts[t] + PUSH_THREADS - 1) / PUSH_THREADS;
-    return (rows + chunk_rows - 1) / chunk_rows;
-  };
+  auto rows = [&](int64_t t) { return (ts[t + 1] - ts[t] + PUSH_THREADS - 1) / PUSH_THREADS; };
   int64_t sa = 0;
-  for (int64_t t = t0; t < t1; t++) sa += chunks(t);
+  for (int64_t t = t0; t < t1; t++) sa += (rows(t) + chunk_rows - 1) / chunk_rows;
   pa[tid] = sa;
   __syncthreads();
   for (int d = 1; d < 1024; d <<= 1) {
@@ -1160,7 +1273,9 @@ __global__ void __launch_bounds__(1024) k_push_chunks(const int64_t* __restrict_
   int64_t ra = pa[tid] - sa;
   for (int64_t t = t0; t < t1; t++) {
     cs[t] = ra;
-    ra += chunks(t);
+    const int64_t r = rows(t);
+    put_chunks(chunks + (int64_t)blockIdx.x * nchunk_max, ra, t, r, tp[t], chunk_rows);
+    ra += (r + chunk_rows - 1) / chunk_rows;
   }
   if (tid == 1023) cs[ntiles] = pa[1023];
 }
@@ -1275,7 +1390,7 @@ __global__ void k_fx_deferred(FxPushArgs a, uint32_t* __restrict__ bits, int64_t
       continue;
     }
     float vx = a.vx[slot], vy = a.vy[slot], vz = a.vz[slot];
-    kick<B>(a, nullptr, nullptr, -1, ib, jb, kb, ps, a.qmp[is], vx, vy, vz);
+    kick<B>(a, nullptr, nullptr, -1, 0, ib, jb, kb, ps.x, ps.y, ps.z, a.qmp[is], vx, vy, vz);
     a.vx[slot] = vx;
     a.vy[slot] = vy;
     a.vz[slot] = vz;
@@ -1292,16 +1407,15 @@ __global__ void k_fx_deferred(FxPushArgs a, uint32_t* __restrict__ bits, int64_t
 inline int fx_box_tile(int tmax) { return tmax <= 4 ? 4 : 8; }
 
 // Dynamic shared memory of the push: int64 accumulator (4 components, or
-// rho alone without the current), row ring, field tile, run queues and cross
-// lists.
+// rho alone without the current), field tile, run queues and lists.
+template <int B>
+constexpr int fx_push_smem_t(bool jd) {
+  const int nf = B * B * B, nbox = ((jd ? 4 : 1) * nf + 1) & ~1;  // as NBOX in k_fx_push
+  return nbox * (int)sizeof(unsigned long long) + FieldT<B>::N * (int)sizeof(float4) + (nf + 1) / 2 * 16 +
+         PUSH_WARPS * (RQCAP * run_words(jd) * (int)sizeof(float) + (XLCAP + OLCAP) * (int)sizeof(int) + RING * ROW32);
+}
 inline int fx_push_smem(int tmax, bool jd = true) {
-  int B = fx_box_tile(tmax) + 2 * PG + 1;
-  int nf = B * B * B;
-  const int qw = (jd ? NJ + NR : NR) + 1;
-  const int nbox = ((jd ? 4 : 1) * nf + 1) & ~1;  // as NBOX in k_fx_push
-  return nbox * (int)sizeof(unsigned long long) + push_stages(jd) * (int)ROW_BYTES +
-         nf * (int)(sizeof(float4) + sizeof(float2)) +
-         PUSH_WARPS * (RQCAP * qw * (int)sizeof(float) + XLCAP * (int)sizeof(int));
+  return fx_box_tile(tmax) == 4 ? fx_push_smem_t<4 + 2 * PG + 1>(jd) : fx_push_smem_t<8 + 2 * PG + 1>(jd);
 }
 
 // The pushing kernel (DEP = true) for a compiled box tile (4 or 8), runs

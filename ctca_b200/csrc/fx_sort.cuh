@@ -37,8 +37,16 @@
 // fixed by the data, so the sort is deterministic, and a particle is read
 // twice (16 bytes to count and rank, 28 to move) and written once (28
 // bytes), plus 4-byte slot indices.  Dead particles and empty slots are
-// dropped (the compaction).  A particle outside its tile's sort box sets the
-// stray flag; the host then sorts with the radix path instead.
+// dropped (the compaction).
+//
+// Strays, particles outside their tile's sort box (fast ones, some per
+// thousand in a hot plasma), are listed by the count pass, sorted by (cell
+// key, slot) by the one block of the tiles pass, and take the ranks after the
+// cell's others.  Without that a single stray sends the whole species to the
+// radix sort, or, inside a CUDA graph, keeps its order for good: the push of
+// a 32^3 x 16 ppc run with strays then took 2.8 times as long.  A
+// species with more than STRAY_MAX of them sets the stray flag; the host then
+// sorts with the radix path instead.
 
 struct LcsGeo {
   int n[3];      // grid cells
@@ -53,6 +61,10 @@ struct LcsGeo {
 // Block size of the per-cell kernels (one thread per cell of a tile of at
 // most 8x8x8 cells).
 constexpr int CELL_THREADS = 512;
+
+// Strays of a species that the tile sort takes (one block sorts them in
+// 128 KB of shared memory).
+constexpr int STRAY_MAX = 16384;
 
 __device__ __forceinline__ int lcs_axis(const LcsGeo& G, int d, int tile, int i) {
   int l = i - (tile * G.t[d] - 1);
@@ -102,11 +114,12 @@ __device__ __forceinline__ void tile_xyz(const Geo& g, int64_t t, int& tx, int& 
 }
 
 // count: per (source tile, warp, box cell).  grid = ntiles, block = PUSH_THREADS.
-__global__ void __launch_bounds__(PUSH_THREADS) k_lcs_count(const float4* __restrict__ pos,
+__global__ void __launch_bounds__(PUSH_THREADS, 2) k_lcs_count(const float4* __restrict__ pos,
                                                             const int64_t* __restrict__ ts,
                                                             const int64_t* __restrict__ tp, Geo g, LcsGeo G,
                                                             uint32_t* __restrict__ wcnt, uint32_t* __restrict__ cnt,
-                                                            int* stray) {
+                                                            int* stray, int* nstray,
+                                                            unsigned long long* __restrict__ slist) {
   extern __shared__ uint32_t hist[];  // [PUSH_WARPS][nbc]
   const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5;
   for (int e = tid; e < PUSH_WARPS * G.nbc; e += PUSH_THREADS) hist[e] = 0;
@@ -127,6 +140,20 @@ __global__ void __launch_bounds__(PUSH_THREADS) k_lcs_count(const float4* __rest
     if (bc < 0) { bad = true; continue; }
     atomicAdd(&hist[warp * G.nbc + bc], 1u);
   }
+  // strays are rare: listed in a pass of their own, by the threads that met one
+  if (bad)
+    for (int r = 0; r < L; r++) {
+      const uint32_t cell = (uint32_t)__float_as_int(src[r * PUSH_THREADS + tid].w);
+      if (cell == DEAD) continue;
+      int i, j, k;
+      unpack(g, cell, i, j, k);
+      if (lcs_box_cell(G, tx, ty, tz, i, j, k) >= 0) continue;
+      const int q = atomicAdd(nstray, 1);
+      if (q < STRAY_MAX)
+        slist[q] = ((unsigned long long)cell_key(g, i, j, k) << 32) | (uint32_t)(tp[t] + r * PUSH_THREADS + tid);
+      else
+        atomicOr(stray, 1);
+    }
   __syncthreads();
   uint32_t* wc = wcnt + (int64_t)t * PUSH_WARPS * G.nbc;
   uint32_t* c = cnt + (int64_t)t * G.nbc;
@@ -139,7 +166,6 @@ __global__ void __launch_bounds__(PUSH_THREADS) k_lcs_count(const float4* __rest
     }
     c[b] = sum;
   }
-  if (bad) atomicOr(stray, 1);
 }
 
 // celltot: per destination cell, the sum over the source tiles holding it;
@@ -184,40 +210,84 @@ __global__ void __launch_bounds__(CELL_THREADS) k_lcs_celltot(const uint32_t* __
 }
 
 // tiles: exclusive scan of the tile totals (one block of 1024 threads):
-// tile_start, tile_pad (whole rows per tile), live count and slot count.
-__global__ void __launch_bounds__(1024) k_lcs_tiles(const int64_t* __restrict__ tiletot, int64_t ntiles,
-                                                    int64_t* ts, int64_t* tp, int64_t* count, int64_t* slots,
-                                                    const int* stray) {
-  __shared__ int64_t pa[1024], pb[1024];
+// tile_start, tile_pad (whole rows per tile), the push's row chunks
+// (chunk_start, as k_push_chunks), live count and slot count.  Before that the
+// strays, sorted (bitonic, in shared memory) and added to the totals.
+__global__ void __launch_bounds__(1024) k_lcs_tiles(int64_t* tiletot, uint32_t* celltot, int64_t ntiles,
+                                                    int64_t* ts, int64_t* tp, int64_t* cs, int4* chunks,
+                                                    int chunk_rows, int64_t* count, int64_t* slots, const int* stray,
+                                                    const int* nstray, unsigned long long* slist, int tcells) {
+  __shared__ int64_t pa[1024], pb[1024], pc[1024];
+  extern __shared__ unsigned long long sl[];  // [STRAY_MAX]
   if (*stray) return;
   const int tid = threadIdx.x;
+  const int ns = *nstray;  // at most STRAY_MAX: the flag is not set
+  if (ns > 0) {
+    int n2 = 1;
+    while (n2 < ns) n2 <<= 1;
+    for (int e = tid; e < n2; e += 1024) sl[e] = e < ns ? slist[e] : ~0ull;
+    __syncthreads();
+    for (int k = 2; k <= n2; k <<= 1)
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        for (int e = tid; e < n2; e += 1024) {
+          const int p = e ^ j;
+          if (p > e) {
+            const unsigned long long x = sl[e], y = sl[p];
+            if ((x > y) == ((e & k) == 0)) {
+              sl[e] = y;
+              sl[p] = x;
+            }
+          }
+        }
+        __syncthreads();
+      }
+    for (int e = tid; e < ns; e += 1024) {
+      const uint32_t key = (uint32_t)(sl[e] >> 32);
+      slist[e] = sl[e];
+      atomicAdd(&celltot[key], 1u);
+      atomicAdd((unsigned long long*)&tiletot[key / (uint32_t)tcells], 1ull);
+    }
+    __threadfence();
+    __syncthreads();
+  }
   const int64_t per = (ntiles + 1023) / 1024;
   const int64_t t0 = tid * per, t1 = min(ntiles, t0 + per);
-  int64_t sa = 0, sb = 0;
+  auto total = [&](int64_t t) { return __ldcg(&tiletot[t]); };
+  auto rows = [&](int64_t t) { return (total(t) + PUSH_THREADS - 1) / PUSH_THREADS; };
+  int64_t sa = 0, sb = 0, sc = 0;
   for (int64_t t = t0; t < t1; t++) {
-    sa += tiletot[t];
-    sb += (tiletot[t] + PUSH_THREADS - 1) / PUSH_THREADS * PUSH_THREADS;
+    const int64_t r = rows(t);
+    sa += total(t);
+    sb += r * PUSH_THREADS;
+    sc += (r + chunk_rows - 1) / chunk_rows;
   }
   pa[tid] = sa;
   pb[tid] = sb;
+  pc[tid] = sc;
   __syncthreads();
   for (int d = 1; d < 1024; d <<= 1) {
-    int64_t va = tid >= d ? pa[tid - d] : 0, vb = tid >= d ? pb[tid - d] : 0;
+    int64_t va = tid >= d ? pa[tid - d] : 0, vb = tid >= d ? pb[tid - d] : 0, vc = tid >= d ? pc[tid - d] : 0;
     __syncthreads();
     pa[tid] += va;
     pb[tid] += vb;
+    pc[tid] += vc;
     __syncthreads();
   }
-  int64_t ra = pa[tid] - sa, rb = pb[tid] - sb;
+  int64_t ra = pa[tid] - sa, rb = pb[tid] - sb, rc = pc[tid] - sc;
   for (int64_t t = t0; t < t1; t++) {
+    const int64_t r = rows(t);
     ts[t] = ra;
     tp[t] = rb;
-    ra += tiletot[t];
-    rb += (tiletot[t] + PUSH_THREADS - 1) / PUSH_THREADS * PUSH_THREADS;
+    cs[t] = rc;
+    put_chunks(chunks, rc, t, r, rb, chunk_rows);
+    ra += total(t);
+    rb += r * PUSH_THREADS;
+    rc += (r + chunk_rows - 1) / chunk_rows;
   }
   if (tid == 1023) {
     ts[ntiles] = pa[1023];
     tp[ntiles] = pb[1023];
+    cs[ntiles] = pc[1023];
     *count = pa[1023];
     *slots = pb[1023];
   }
@@ -229,7 +299,8 @@ __global__ void __launch_bounds__(CELL_THREADS) k_lcs_bases(const uint32_t* __re
                                                             uint32_t* celltot, Geo g, LcsGeo G,
                                                             const int64_t* __restrict__ ts,
                                                             const int64_t* __restrict__ tp, uint32_t* __restrict__ base,
-                                                            uint32_t* __restrict__ inv, const int* stray) {
+                                                            uint32_t* __restrict__ inv, const int* stray,
+                                                            const int* nstray, uint32_t* __restrict__ regend) {
   __shared__ uint32_t sc[CELL_THREADS];
   if (*stray) return;
   const int t = blockIdx.x, tid = threadIdx.x;
@@ -262,6 +333,8 @@ __global__ void __launch_bounds__(CELL_THREADS) k_lcs_bases(const uint32_t* __re
             base[tt * G.nbc + bc] = run;
             run += cnt[tt * G.nbc + bc];
           }
+      // the strays of the cell come next
+      if (*nstray) regend[(int64_t)t * G.tcells + tid] = run;
     }
     // the cell's end rank (its tail particles take the ranks before it)
     celltot[(int64_t)t * G.tcells + tid] = (uint32_t)ts[t] + sc[tid];
@@ -291,7 +364,7 @@ __device__ __forceinline__ uint32_t fastdiv(uint32_t q, uint32_t d, uint64_t M) 
 // regions; inv[new slot] = old slot (4-byte scattered writes).  grid =
 // ntiles, block = PUSH_THREADS, shared = PUSH_WARPS * nbc * 4.
 
-__global__ void __launch_bounds__(PUSH_THREADS) k_lcs_rank(const float4* __restrict__ pos,
+__global__ void __launch_bounds__(PUSH_THREADS, 2) k_lcs_rank(const float4* __restrict__ pos,
                                                               const int64_t* __restrict__ ts,
                                                               const int64_t* __restrict__ tp, Geo g, LcsGeo G,
                                                               const uint32_t* __restrict__ wcnt,
@@ -299,7 +372,9 @@ __global__ void __launch_bounds__(PUSH_THREADS) k_lcs_rank(const float4* __restr
                                                               const int64_t* __restrict__ ts2,
                                                               const int64_t* __restrict__ tp2,
                                                               uint32_t* __restrict__ inv, int* status,
-                                                              long long* diag, const int* stray) {
+                                                              long long* diag, const int* stray, const int* nstray,
+                                                              const unsigned long long* __restrict__ slist,
+                                                              const uint32_t* __restrict__ regend) {
   extern __shared__ uint32_t wb[];  // [PUSH_WARPS][nbc] next rank of (warp, box cell)
   if (*stray) return;
   const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -357,6 +432,7 @@ __global__ void __launch_bounds__(PUSH_THREADS) k_lcs_rank(const float4* __restr
             ext2 = min(G.t[2], G.n[2] - tz * G.t[2]);
   // the cells of the next rows are loaded ahead
   constexpr int AHEAD = 4;
+  bool bad = false;  // this thread met a stray
   uint32_t cr[AHEAD];
 #pragma unroll
   for (int q = 0; q < AHEAD; q++)
@@ -372,10 +448,12 @@ __global__ void __launch_bounds__(PUSH_THREADS) k_lcs_rank(const float4* __restr
       int i, j, k;
       unpack(g, cell, i, j, k);
       const int a = lcs_axis(G, 0, tx, i), b = lcs_axis(G, 1, ty, j), c = lcs_axis(G, 2, tz, k);
-      if ((a | b | c) >= 0) {  // else a stray: the radix path sorts
+      if ((a | b | c) >= 0) {
         bc = a + G.bc[0] * (b + G.bc[1] * c);
         nb = (a == 0 ? 0 : (a <= ext0 ? 1 : 2)) + 3 * (b == 0 ? 0 : (b <= ext1 ? 1 : 2)) +
              9 * (c == 0 ? 0 : (c <= ext2 ? 1 : 2));
+      } else {
+        bad = true;
       }
     }
     const unsigned peers = __match_any_sync(0xffffffffu, bc);
@@ -393,6 +471,33 @@ __global__ void __launch_bounds__(PUSH_THREADS) k_lcs_rank(const float4* __restr
     const uint32_t Ld = nld[nb];
     const uint32_t col = fastdiv(q, Ld, nmul[nb]);
     inv[ntp[nb] + (q - col * Ld) * PUSH_THREADS + col] = (uint32_t)m;
+  }
+  if (!bad) return;
+  // strays: their places among the cell's strays, after the cell's others
+  const int ns = *nstray;
+  auto below = [&](unsigned long long v) {  // entries less than v
+    int lo = 0, hi = ns;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (slist[mid] < v) lo = mid + 1;
+      else hi = mid;
+    }
+    return lo;
+  };
+  for (int r = 0; r < L; r++) {
+    const int64_t m = s0 + (int64_t)r * PUSH_THREADS + tid;
+    const uint32_t cell = (uint32_t)__float_as_int(pos[m].w);
+    if (cell == DEAD) continue;
+    int i, j, k;
+    unpack(g, cell, i, j, k);
+    if (lcs_box_cell(G, tx, ty, tz, i, j, k) >= 0) continue;
+    const unsigned long long first = (unsigned long long)cell_key(g, i, j, k) << 32;
+    const uint32_t key = (uint32_t)(first >> 32);
+    const int64_t td = key / (uint32_t)G.tcells;
+    const int64_t q = (int64_t)regend[key] + (below(first | (uint32_t)m) - below(first)) - ts2[td];
+    const int64_t nd = ts2[td + 1] - ts2[td], Ld = (nd + PUSH_THREADS - 1) / PUSH_THREADS;
+    if (q < 0 || q >= nd) report_bad(status, diag, SITE_FX_SORT, m, (long long)cell);
+    else inv[tp2[td] + (q % Ld) * PUSH_THREADS + q / Ld] = (uint32_t)m;
   }
 }
 
@@ -439,18 +544,6 @@ template <class Cfg>
 inline int move_smem() { return Cfg::NBUF * Cfg::BUF; }
 static_assert(PUSH_THREADS % 32 == 0, "32-column groups divide the row");
 
-template <bool CA>
-__device__ __forceinline__ void cpa16(void* dst, const void* src) {
-  if (CA)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-  else
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cpa_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
 __device__ __forceinline__ bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // One destination tile with groups of GW columns (see k_lcs_move).
@@ -628,13 +721,14 @@ __global__ void __launch_bounds__(PUSH_THREADS, 1) k_lcs_move(const float4* __re
   move_tile<Cfg, 32>(pos, vx, vy, vz, inv, pos2, vx2, vy2, vz2, Ld, Ls, tp[t], tp2[t], ns > 0, msm, wlo);
 }
 
-// Inside a CUDA graph the host cannot switch to the radix sort when a
-// particle has left its tile's sort box; the sort kernels above then return
+// Inside a CUDA graph the host cannot switch to the radix sort when more
+// than STRAY_MAX particles of a species have left their sort boxes; the sort
+// kernels above then return
 // at once and this one keeps the current order instead: the new buffers get
 // the old regions slot for slot (inv = identity).  The push handles a
 // particle outside its tile's box on its general path (global gather and
 // deposits), so the step stays correct, only slower, until the next sort
-// outside a graph.  Does nothing when no particle strayed.
+// outside a graph.  Does nothing when the sort went through.
 __global__ void __launch_bounds__(256) k_lcs_keep(const int* stray, const float4* __restrict__ pos,
                                                   const float* __restrict__ vx, const float* __restrict__ vy,
                                                   const float* __restrict__ vz, const int64_t* __restrict__ ts,

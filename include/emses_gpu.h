@@ -329,8 +329,9 @@ int emsesg_upload_field_async(emsesg_ctx* ctx, int field, const double* host);
  * (emsesg_fx_step with do_sort on every sort_every-th step).  With use_graph,
  * a block of 2*sort_every steps is captured once into a CUDA graph (cached
  * per ustep and sort_every) and replayed; the remaining steps run one by one.
- * Inside the graph a tile sort that meets a particle outside its tile's sort
- * box cannot switch to the global sort: it keeps the current order for that
+ * Inside the graph a tile sort that meets more than 16384 particles of a
+ * species outside their tiles' sort boxes (fewer it takes along) cannot switch
+ * to the global sort: it keeps the current order for that
  * species (the push handles such particles on its general path), so rho/J
  * stay the same physics, though their FP32 partial sums may round in a
  * different order than emsesg_fx_step's.  Injected particles waiting in the
