@@ -25,6 +25,19 @@ struct FieldDesc {
   __host__ __device__ int64_t size() const { return (int64_t)nc * ex * ey * ez; }
 };
 
+// Node t of an ex x ey x ... array, x fastest, in 32 bits: arrays of 2^32
+// nodes do not fit the device (eb alone takes 48 bytes a node), and 64-bit
+// divisions take several times as long (the grid kernels of an electrostatic
+// step, 64 x 64 x 70 cells with plates: 3 % of the step).
+struct Node3 {
+  int i, j, k;
+};
+__host__ __device__ inline Node3 node3(int64_t t, int64_t ex, int64_t ey) {
+  const uint32_t u = (uint32_t)t, x = (uint32_t)ex, y = (uint32_t)ey;
+  const uint32_t row = u / x, plane = row / y;
+  return Node3{(int)(u - row * x), (int)(row - plane * y), (int)plane};
+}
+
 // Guard extents from OhHelp's fsizes rule (ohhelp3.c:439-477) applied to
 // ftypes/ctypes of src/wrapper/ohinit.F90:98-122.
 FieldDesc field_desc(const emsesg_config& c, int field);

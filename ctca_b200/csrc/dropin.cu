@@ -658,7 +658,8 @@ __global__ void k_flush_tj(const double* __restrict__ tj, double* aj, double* aj
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t ex = nx + 3, ey = ny + 3, ez = nz + 3;
   if (t >= ex * ey * ez) return;
-  int i = (int)(t % ex) - 1, j = (int)((t / ex) % ey) - 1, k = (int)(t / (ex * ey)) - 1;
+  const Node3 at = node3(t, ex, ey);
+  const int i = at.i - 1, j = at.j - 1, k = at.k - 1;
   for (int d = 0; d < 3; d++) {
     double v = tj[fa.at(d, i, j, k)];
     aj[fa.at(d, i, j, k)] = aj[fa.at(d, i, j, k)] + v * qs;
@@ -684,7 +685,8 @@ __global__ void k_grdcrt(const double* __restrict__ eb, double* __restrict__ nod
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t ex = nx + 1, ey = ny + 1, ez = nz + 1;
   if (t >= ex * ey * ez) return;
-  int i = (int)(t % ex), j = (int)((t / ex) % ey), k = (int)(t / (ex * ey));
+  const Node3 at = node3(t, ex, ey);
+  const int i = at.i, j = at.j, k = at.k;
   double* o = node + 8 * ((int64_t)i + (ex + 1) * ((int64_t)j + (ey + 1) * k));
   o[EX] = 0.5 * (eb[fe.at(EX, i, j, k)] + eb[fe.at(EX, i - 1, j, k)]) + e0x;
   o[EY] = 0.5 * (eb[fe.at(EY, i, j, k)] + eb[fe.at(EY, i, j - 1, k)]) + e0y;
@@ -704,7 +706,8 @@ __global__ void k_node_to_wrk(const double* __restrict__ node, double* wrk, Fiel
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t ex = nx + 1, ey = ny + 1, ez = nz + 1;
   if (t >= ex * ey * ez) return;
-  int i = (int)(t % ex), j = (int)((t / ex) % ey), k = (int)(t / (ex * ey));
+  const Node3 at = node3(t, ex, ey);
+  const int i = at.i, j = at.j, k = at.k;
   int64_t nd = (int64_t)i + (ex + 1) * ((int64_t)j + (ey + 1) * k);
   for (int cc = 0; cc < 6; cc++) wrk[fw.at(cc, i, j, k)] = node[8 * nd + cc];
 }
@@ -796,7 +799,8 @@ __global__ void k_rhoupd(double* rho, const double* __restrict__ aj, FieldDesc f
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t ex = nx + 1, ey = ny + 1, ez = nz + 1;
   if (t >= ex * ey * ez) return;
-  int i = (int)(t % ex), j = (int)((t / ex) % ey), k = (int)(t / (ex * ey));
+  const Node3 at = node3(t, ex, ey);
+  const int i = at.i, j = at.j, k = at.k;
   rho[fr.at(0, i, j, k)] = rho[fr.at(0, i, j, k)] -
       (aj[fa.at(JX, i, j, k)] - aj[fa.at(JX, i - 1, j, k)] + aj[fa.at(JY, i, j, k)] - aj[fa.at(JY, i, j - 1, k)] +
        aj[fa.at(JZ, i, j, k)] - aj[fa.at(JZ, i, j, k - 1)]) * 2.0;
@@ -808,7 +812,8 @@ __global__ void k_bfield(double* eb, FieldDesc f, int nx, int ny, int nz) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t ex = nx + 2, ey = ny + 2, ez = nz + 2;
   if (t >= ex * ey * ez) return;
-  const int i = (int)(t % ex) - 1, j = (int)((t / ex) % ey) - 1, k = (int)(t / (ex * ey)) - 1;
+  const Node3 at = node3(t, ex, ey);
+  const int i = at.i - 1, j = at.j - 1, k = at.k - 1;
   eb[f.at(BX, i, j, k)] = eb[f.at(BX, i, j, k)] + eb[f.at(EY, i, j, k + 1)] - eb[f.at(EY, i, j, k)] -
                           eb[f.at(EZ, i, j + 1, k)] + eb[f.at(EZ, i, j, k)];
   eb[f.at(BY, i, j, k)] = eb[f.at(BY, i, j, k)] + eb[f.at(EZ, i + 1, j, k)] - eb[f.at(EZ, i, j, k)] -
@@ -824,7 +829,8 @@ __global__ void k_efield(double* eb, const double* __restrict__ aj, FieldDesc f,
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t ex = nx + 1, ey = ny + 1, ez = nz + 1;
   if (t >= ex * ey * ez) return;
-  const int i = (int)(t % ex), j = (int)((t / ex) % ey), k = (int)(t / (ex * ey));
+  const Node3 at = node3(t, ex, ey);
+  const int i = at.i, j = at.j, k = at.k;
   eb[f.at(EX, i, j, k)] = eb[f.at(EX, i, j, k)] +
                           tcs * (eb[f.at(BZ, i, j, k)] - eb[f.at(BZ, i, j - 1, k)] - eb[f.at(BY, i, j, k)] +
                                  eb[f.at(BY, i, j, k - 1)]) -

@@ -52,7 +52,8 @@ __global__ void k_es_pack(const double* __restrict__ rho, FieldDesc fr, int nx, 
                           double* __restrict__ r) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)nx * ny * nz) return;
-  const int i = (int)(t % nx), j = (int)((t / nx) % ny), k = (int)(t / ((int64_t)nx * ny));
+  const Node3 at = node3(t, nx, ny);
+  const int i = at.i, j = at.j, k = at.k;
   r[t] = rho[fr.at(0, i, j, k)];
 }
 
@@ -63,7 +64,8 @@ __global__ void k_es_divide(cufftDoubleComplex* __restrict__ c, const double* __
                             double mfactor) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)nxh * ny * nz) return;
-  const int i = (int)(t % nxh), j = (int)((t / nxh) % ny), k = (int)(t / ((int64_t)nxh * ny));
+  const Node3 at = node3(t, nxh, ny);
+  const int i = at.i, j = at.j, k = at.k;
   const double divisor = (lx[i] + ly[j] + lz[k]) * mfactor;
   cufftDoubleComplex v = c[t];
   if (divisor != 0.0) {
@@ -84,7 +86,8 @@ __global__ void k_es_unpack(const double* __restrict__ p, double* __restrict__ p
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int ex = nx + 3, ey = ny + 3, ez = nz + 3;
   if (t >= (int64_t)ex * ey * ez) return;
-  const int i = (int)(t % ex) - 1, j = (int)((t / ex) % ey) - 1, k = (int)(t / ((int64_t)ex * ey)) - 1;
+  const Node3 at = node3(t, ex, ey);
+  const int i = at.i - 1, j = at.j - 1, k = at.k - 1;
   const int si = (i + nx) % nx, sj = (j + ny) % ny, sk = (k + nz) % nz;
   phi[fp.at(0, i, j, k)] = p[si + (int64_t)nx * (sj + (int64_t)ny * sk)];
 }
@@ -97,8 +100,8 @@ __global__ void k_es_efield(const double* __restrict__ phi, FieldDesc fp, double
                             int nx, int ny, int nz, double mlt, int tx, int ty, int tz) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)fe.ex * fe.ey * fe.ez) return;
-  const int i = (int)(t % fe.ex) + fe.lo, j = (int)((t / fe.ex) % fe.ey) + fe.lo,
-            k = (int)(t / ((int64_t)fe.ex * fe.ey)) + fe.lo;
+  const Node3 at = node3(t, fe.ex, fe.ey);
+  const int i = at.i + fe.lo, j = at.j + fe.lo, k = at.k + fe.lo;
   const bool jk = j >= 0 && j <= ny && k >= 0 && k <= nz;
   const bool ik = i >= 0 && i <= nx && k >= 0 && k <= nz;
   const bool ij = i >= 0 && i <= nx && j >= 0 && j <= ny;
@@ -135,7 +138,8 @@ __global__ void k_es_poichk(const double* __restrict__ rho, FieldDesc fr, const 
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   double d2 = 0.0;
   if (t < (int64_t)cx * cy * cz) {
-    const int i = x0 + (int)(t % cx), j = y0 + (int)((t / cx) % cy), k = z0 + (int)(t / ((int64_t)cx * cy));
+    const Node3 at = node3(t, cx, cy);
+    const int i = x0 + at.i, j = y0 + at.j, k = z0 + at.k;
     const double drho = rho[fr.at(0, i, j, k)] +
                         (phi[fp.at(0, i - 1, j, k)] + phi[fp.at(0, i + 1, j, k)] + phi[fp.at(0, i, j - 1, k)] +
                          phi[fp.at(0, i, j + 1, k)] + phi[fp.at(0, i, j, k - 1)] + phi[fp.at(0, i, j, k + 1)]) -
@@ -168,8 +172,8 @@ struct EsBc {
 __global__ void k_es_pack_w(const double* __restrict__ rho, FieldDesc fr, EsGeo G, EsBc bc, double* __restrict__ w) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)G.m[0] * G.m[1] * G.m[2]) return;
-  const int nd[3] = {G.lo[0] + (int)(t % G.m[0]), G.lo[1] + (int)((t / G.m[0]) % G.m[1]),
-                     G.lo[2] + (int)(t / ((int64_t)G.m[0] * G.m[1]))};
+  const Node3 at = node3(t, G.m[0], G.m[1]);
+  const int nd[3] = {G.lo[0] + at.i, G.lo[1] + at.j, G.lo[2] + at.k};
   double v = rho[fr.at(0, nd[0], nd[1], nd[2])];
   for (int d = 0; d < 3; d++) {
     if (G.t[d] != 2) continue;
@@ -185,9 +189,15 @@ __device__ __forceinline__ int64_t es_widx(const EsGeo& G, int a, int64_t l, int
   const int p = a == 0 ? 1 : 0, q = a == 2 ? 1 : 2;
   int id[3];
   id[a] = u;
-  id[p] = (int)(l % G.m[p]);
-  id[q] = (int)(l / G.m[p]);
+  id[q] = (int)((uint32_t)l / (uint32_t)G.m[p]);
+  id[p] = (int)((uint32_t)l - (uint32_t)id[q] * (uint32_t)G.m[p]);
   return id[0] + (int64_t)G.m[0] * (id[1] + (int64_t)G.m[1] * id[2]);
+}
+
+// t / L, in 32 bits where t fits (the extended lines of a grid near the
+// device's memory may have more elements).
+__device__ __forceinline__ int64_t line_of(int64_t t, int L) {
+  return t < (1LL << 32) ? (int64_t)((uint32_t)t / (uint32_t)L) : t / L;
 }
 
 // Line transforms of axis a (kind 0: R2HC, 1: HC2R, 2: RODFT00, 3: REDFT00):
@@ -196,8 +206,8 @@ __global__ void k_es_line_in(const double* __restrict__ w, EsGeo G, int a, int k
                              cufftDoubleComplex* __restrict__ z) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= lines * L) return;
-  const int64_t l = t / L;
-  const int u = (int)(t % L), n = G.n[a];
+  const int64_t l = line_of(t, L);
+  const int u = (int)(t - l * L), n = G.n[a];
   double re = 0.0, im = 0.0;
   if (kind == 0) {
     re = w[es_widx(G, a, l, u)];
@@ -229,8 +239,8 @@ __global__ void k_es_line_out(const cufftDoubleComplex* __restrict__ z, EsGeo G,
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int m = G.m[a], n = G.n[a];
   if (t >= lines * m) return;
-  const int64_t l = t / m;
-  const int u = (int)(t % m);
+  const int64_t l = line_of(t, m);
+  const int u = (int)(t - l * m);
   const cufftDoubleComplex* zl = z + l * L;
   double v;
   if (kind == 0) v = 2 * u <= n ? zl[u].x : zl[n - u].y;
@@ -245,7 +255,8 @@ __global__ void k_es_divide_w(double* __restrict__ w, const double* __restrict__
                               const double* __restrict__ lz, EsGeo G, double mfactor) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)G.m[0] * G.m[1] * G.m[2]) return;
-  const int i = (int)(t % G.m[0]), j = (int)((t / G.m[0]) % G.m[1]), k = (int)(t / ((int64_t)G.m[0] * G.m[1]));
+  const Node3 at = node3(t, G.m[0], G.m[1]);
+  const int i = at.i, j = at.j, k = at.k;
   const double divisor = (lx[i] + ly[j] + lz[k]) * mfactor;
   w[t] = divisor != 0.0 ? w[t] / divisor : 0.0;
 }
@@ -256,7 +267,8 @@ __global__ void k_es_unpack_w(const double* __restrict__ w, double* __restrict__
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int ex = G.n[0] + 3, ey = G.n[1] + 3, ez = G.n[2] + 3;
   if (t >= (int64_t)ex * ey * ez) return;
-  const int nd[3] = {(int)(t % ex) - 1, (int)((t / ex) % ey) - 1, (int)(t / ((int64_t)ex * ey)) - 1};
+  const Node3 at = node3(t, ex, ey);
+  const int nd[3] = {at.i - 1, at.j - 1, at.k - 1};
   int id[3];
   bool in = true;
   for (int d = 0; d < 3; d++) {

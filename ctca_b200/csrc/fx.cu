@@ -75,7 +75,8 @@ __global__ void k_grdcrt32(const double* __restrict__ eb, float4* __restrict__ f
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t ex = nx + 1, ey = ny + 1;
   if (t >= ex * ey * nk) return;
-  int i = (int)(t % ex), j = (int)((t / ex) % ey), k = k0 + (int)(t / (ex * ey));
+  const Node3 n3 = node3(t, ex, ey);
+  const int i = n3.i, j = n3.j, k = k0 + n3.k;
   t += (int64_t)k0 * ex * ey;
   double wex = 0.5 * (eb[fe.at(0, i, j, k)] + eb[fe.at(0, i - 1, j, k)]) + e0x;
   double wey = 0.5 * (eb[fe.at(1, i, j, k)] + eb[fe.at(1, i, j - 1, k)]) + e0y;
@@ -530,12 +531,16 @@ int fx_alloc(emsesg_ctx* ctx) {
     const int lsm = (int)(PUSH_WARPS * 10 * 10 * 10 * sizeof(uint32_t));
     EMSESG_CUDA(ctx, cudaFuncSetAttribute(k_lcs_count, cudaFuncAttributeMaxDynamicSharedMemorySize, lsm));
     EMSESG_CUDA(ctx, cudaFuncSetAttribute(k_lcs_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, lsm));
-    EMSESG_CUDA(ctx, cudaFuncSetAttribute(k_lcs_move<MoveBig>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          move_smem<MoveBig>()));
-    EMSESG_CUDA(ctx, cudaFuncSetAttribute(k_lcs_move<MoveSmall>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          move_smem<MoveSmall>()));
-    EMSESG_CUDA(ctx, cudaFuncSetAttribute(k_lcs_move<MoveMid>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          move_smem<MoveMid>()));
+    auto move_attr = [&](auto cfg) {
+      using Cfg = decltype(cfg);
+      EMSESG_CUDA(ctx, cudaFuncSetAttribute(k_lcs_move<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            move_smem<Cfg>()));
+      return (int)EMSESG_OK;
+    };
+    int arc;
+    if ((arc = move_attr(MoveBig())) || (arc = move_attr(MoveMid())) || (arc = move_attr(MoveSmall())) ||
+        (arc = move_attr(MoveMidMany())) || (arc = move_attr(MoveSmallMany())))
+      return arc;
   }
   EMSESG_CUDA(ctx, cudaFuncSetAttribute(k_fx_push<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         fx_push_smem(4)));
@@ -684,19 +689,24 @@ int fx_local_sort(emsesg_ctx* ctx, bool* done) {
       EMSESG_LAUNCH(ctx, "lcs_tail_inv", k_lcs_tail_inv, nblk(nt), 256, 0, tk, tv, nt, deadkey, (int)tcells,
                     f.lcs_celltot, ts2, tp2, f.lcs_inv + off, stray);
     // the move's shape from the mean rows per tile (the host's count is an
-    // upper bound between synchronisations: escapes are not in it)
-    if (ctx->totalp[is] + nt <= (int64_t)MOVE_SMALL_ROWS * PUSH_THREADS * f.ntiles)
-      EMSESG_LAUNCH(ctx, "lcs_move", k_lcs_move<MoveSmall>, (unsigned)f.ntiles, PUSH_THREADS, move_smem<MoveSmall>(),
-                    f.pos + off, f.vx + off, f.vy + off, f.vz + off, f.tile_start + is * T1, f.tile_pad + is * T1, ts2,
-                    tp2, f.lcs_inv + off, f.pos2 + off, f.vx2 + off, f.vy2 + off, f.vz2 + off, stray);
-    else if (ctx->totalp[is] + nt <= (int64_t)MOVE_MID_ROWS * PUSH_THREADS * f.ntiles)
-      EMSESG_LAUNCH(ctx, "lcs_move", k_lcs_move<MoveMid>, (unsigned)f.ntiles, PUSH_THREADS, move_smem<MoveMid>(),
-                    f.pos + off, f.vx + off, f.vy + off, f.vz + off, f.tile_start + is * T1, f.tile_pad + is * T1, ts2,
-                    tp2, f.lcs_inv + off, f.pos2 + off, f.vx2 + off, f.vy2 + off, f.vz2 + off, stray);
+    // upper bound between synchronisations: escapes are not in it) and the
+    // number of tiles
+    auto move = [&](auto cfg) {
+      using Cfg = decltype(cfg);
+      EMSESG_LAUNCH(ctx, "lcs_move", k_lcs_move<Cfg>, (unsigned)f.ntiles, Cfg::T, move_smem<Cfg>(), f.pos + off,
+                    f.vx + off, f.vy + off, f.vz + off, f.tile_start + is * T1, f.tile_pad + is * T1, ts2, tp2,
+                    f.lcs_inv + off, f.pos2 + off, f.vx2 + off, f.vy2 + off, f.vz2 + off, stray);
+      return (int)EMSESG_OK;
+    };
+    const int64_t mean = ctx->totalp[is] + nt, per_row = PUSH_THREADS * f.ntiles;
+    int mrc;
+    if (mean <= MOVE_SMALL_ROWS * per_row)
+      mrc = f.ntiles >= MOVE_SMALL_TILES ? move(MoveSmallMany()) : move(MoveSmall());
+    else if (mean <= MOVE_MID_ROWS * per_row)
+      mrc = f.ntiles >= MOVE_MID_TILES ? move(MoveMidMany()) : move(MoveMid());
     else
-      EMSESG_LAUNCH(ctx, "lcs_move", k_lcs_move<MoveBig>, (unsigned)f.ntiles, PUSH_THREADS, move_smem<MoveBig>(),
-                    f.pos + off, f.vx + off, f.vy + off, f.vz + off, f.tile_start + is * T1, f.tile_pad + is * T1, ts2,
-                    tp2, f.lcs_inv + off, f.pos2 + off, f.vx2 + off, f.vy2 + off, f.vz2 + off, stray);
+      mrc = move(MoveBig());
+    if (mrc) return mrc;
     if (f.capture)
       EMSESG_LAUNCH(ctx, "lcs_keep", k_lcs_keep, 4 * 148, 256, 0, stray, f.pos + off, f.vx + off, f.vy + off,
                     f.vz + off, f.tile_start + is * T1, f.tile_pad + is * T1, f.ntiles, f.pos2 + off, f.vx2 + off,

@@ -522,23 +522,35 @@ __global__ void __launch_bounds__(PUSH_THREADS, 2) k_lcs_rank(const float4* __re
 // z (whose rank moves by a z-layer, tens of columns) are found there.
 // A third shape (MoveMid) for tiles of up to 56 rows keeps two groups'
 // copies in flight (three buffers) while one group is written.
-// grid = ntiles, block = PUSH_THREADS (one CTA per SM), shared =
-// Cfg::NBUF * Cfg::BUF.
-template <int WIN_, int SLOTS_, bool CA_, int NBUF_ = 2>
+// grid = ntiles, block = Cfg::T, shared = Cfg::NBUF * Cfg::BUF.
+template <int WIN_, int SLOTS_, bool CA_, int NBUF_, int T_, int CTAS_>
 struct MoveCfg {
+  static constexpr int T = T_;          // threads of a CTA
+  static constexpr int CTAS = CTAS_;    // CTAs of a multiprocessor
   static constexpr int WIN = WIN_;      // window particles of one buffer
   static constexpr int SLOTS = SLOTS_;  // slots of one group (staged inv)
   static constexpr bool CA = CA_;       // copies cached in L1
   static constexpr int NBUF = NBUF_;    // buffers: NBUF - 1 groups in flight while one is written
-  static constexpr int K = (SLOTS + PUSH_THREADS - 1) / PUSH_THREADS;  // slots of a thread per group
+  static constexpr int K = (SLOTS + T - 1) / T;  // slots of a thread per group
   static constexpr int BUF = WIN * (16 + 3 * 4) + SLOTS * 4;          // bytes of one buffer
-  static_assert(NBUF == 2 || NBUF == 3, "double or triple buffering");
+  static_assert(NBUF >= 1 && NBUF <= 3, "one to three buffers");
 };
-using MoveBig = MoveCfg<3200, 2560, false>;      // up to 80 rows of 40 columns
-using MoveMid = MoveCfg<2240, 1792, false, 3>;   // up to 56 rows of 40 columns, two groups in flight
-using MoveSmall = MoveCfg<1600, 1280, true>;     // up to 40 rows of 40 columns
+using MoveBig = MoveCfg<3200, 2560, false, 2, PUSH_THREADS, 1>;      // up to 80 rows of 40 columns
+using MoveMid = MoveCfg<2240, 1792, false, 3, PUSH_THREADS, 1>;   // up to 56 rows of 40 columns, two groups in flight
+using MoveSmall = MoveCfg<1600, 1280, true, 2, PUSH_THREADS, 1>;     // up to 40 rows of 40 columns
+// With many tiles, one buffer and three CTAs of fewer threads a multiprocessor:
+// the other CTAs' copies and writes fill the waits, and no barrier holds 23
+// warps.  Small, per species: 75x42x61 x 40/20 ppc (480 tiles) 177 -> 136 us,
+// 80x64x96 x 32 ppc (960) 343 -> 286; with 64 tiles (32^3 x 16 ppc) the fewer
+// threads of a tile show, 39 -> 50, so it starts where the tiles fill all the
+// CTAs once.  Mid: 128^3 x 64 ppc (4096 tiles) 2.32 -> 2.12 ms; 64^3 (512) 0.34
+// -> 0.39, so four times that.
+using MoveSmallMany = MoveCfg<1600, 1280, true, 1, 384, 3>;
+using MoveMidMany = MoveCfg<1920, 1536, false, 1, 256, 3>;  // up to 48 rows of 40 columns
 constexpr int MOVE_SMALL_ROWS = 32;              // mean rows per tile up to which MoveSmall is used
 constexpr int MOVE_MID_ROWS = 48;                // then MoveMid up to this mean
+constexpr int MOVE_SMALL_TILES = 3 * 148;        // tiles from which the ...Many shapes are used
+constexpr int MOVE_MID_TILES = 4 * 3 * 148;
 constexpr int MOVE_MAXGROUPS = PUSH_THREADS / 32;
 template <class Cfg>
 inline int move_smem() { return Cfg::NBUF * Cfg::BUF; }
@@ -582,31 +594,34 @@ __device__ __forceinline__ void move_tile(const float4* __restrict__ pos, const 
     if (win) {
       const int lo = wlo[grp];
       const float4* ps = pos + sbase + lo;
-      for (int e = tid; e < Ls * WC; e += PUSH_THREADS) {
+      for (int e = tid; e < Ls * WC; e += Cfg::T) {
         const int row = e / WC, col = e - row * WC;
         cpa16<Cfg::CA>(wpos + e, ps + row * PUSH_THREADS + col);
       }
       const float* v3[3] = {vx + sbase + lo, vy + sbase + lo, vz + sbase + lo};
 #pragma unroll
       for (int arr = 0; arr < 3; arr++)
-        for (int h = tid; h < Ls * VCH; h += PUSH_THREADS) {
+        for (int h = tid; h < Ls * VCH; h += Cfg::T) {
           const int row = h / VCH, ch = h - row * VCH;
           cpa16<Cfg::CA>(wv + arr * MOVE_WIN + row * WC + 4 * ch, v3[arr] + row * PUSH_THREADS + 4 * ch);
         }
     }
     if (sinv) {
       const uint32_t* is = inv + d0 + grp * GW;
-      for (int e = tid; e < Ld * GCH; e += PUSH_THREADS) {
+      for (int e = tid; e < Ld * GCH; e += Cfg::T) {
         const int row = e / GCH, ch = e - row * GCH;
         cpa16<Cfg::CA>(winv + row * GW + 4 * ch, is + row * PUSH_THREADS + 4 * ch);
       }
     }
     cpa_commit();
   };
-  stage(0);
+  if (Cfg::NBUF > 1) stage(0);
   if (Cfg::NBUF == 3 && NG > 1) stage(1);
   for (int grp = 0; grp < NG; grp++) {
-    if (Cfg::NBUF == 3) {
+    if (Cfg::NBUF == 1) {
+      stage(grp);
+      cpa_wait<0>();
+    } else if (Cfg::NBUF == 3) {
       if (grp + 2 < NG) {
         stage(grp + 2);
         cpa_wait<2>();
@@ -633,12 +648,12 @@ __device__ __forceinline__ void move_tile(const float4* __restrict__ pos, const 
     // MOVE_K slots of a thread at a time (all of the group's when its inv is
     // staged): every load is issued before the first store, so the
     // particles gathered from global memory are in flight together
-    for (int e0 = 0; e0 < Ld * GW; e0 += MOVE_K * PUSH_THREADS) {
+    for (int e0 = 0; e0 < Ld * GW; e0 += MOVE_K * Cfg::T) {
       float4 p[MOVE_K];
       float a[MOVE_K], b[MOVE_K], c[MOVE_K];
 #pragma unroll
       for (int k = 0; k < MOVE_K; k++) {
-        const int e = e0 + tid + k * PUSH_THREADS;
+        const int e = e0 + tid + k * Cfg::T;
         p[k] = make_float4(0.f, 0.f, 0.f, __int_as_float((int)DEAD));
         a[k] = b[k] = c[k] = 0.f;
         if (e < Ld * GW) {
@@ -665,7 +680,7 @@ __device__ __forceinline__ void move_tile(const float4* __restrict__ pos, const 
       }
 #pragma unroll
       for (int k = 0; k < MOVE_K; k++) {
-        const int e = e0 + tid + k * PUSH_THREADS;
+        const int e = e0 + tid + k * Cfg::T;
         if (e < Ld * GW) {
           const int row = e / GW;
           const int64_t m = g0 + (int64_t)row * PUSH_THREADS + (e - row * GW);
@@ -681,7 +696,7 @@ __device__ __forceinline__ void move_tile(const float4* __restrict__ pos, const 
 }
 
 template <class Cfg>
-__global__ void __launch_bounds__(PUSH_THREADS, 1) k_lcs_move(const float4* __restrict__ pos,
+__global__ void __launch_bounds__(Cfg::T, Cfg::CTAS) k_lcs_move(const float4* __restrict__ pos,
                                                               const float* __restrict__ vx,
                                                               const float* __restrict__ vy,
                                                               const float* __restrict__ vz,
