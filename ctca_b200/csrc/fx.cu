@@ -649,7 +649,7 @@ int fx_local_sort(emsesg_ctx* ctx, bool* done) {
     // per-warp counts (one species at a time)
     EMSESG_LAUNCH(ctx, "lcs_count", k_lcs_count, (unsigned)f.ntiles, PUSH_THREADS, lsm, f.pos + off,
                   f.tile_start + is * T1, f.tile_pad + is * T1, g, G[is], f.lcs_wcnt, cnt, f.lcs_stray + is, nstray,
-                  f.lcs_slist);
+                  f.lcs_slist, ctx->d_status, ctx->d_diag);
     // Outside a stream capture the host reads the flag of too many strays and
     // falls back to the radix sort (which redoes every species).  Inside one
     // (emsesg_fx_run's graph) it cannot: the sort kernels of such a species

@@ -727,7 +727,8 @@ __device__ __forceinline__ int body_absorb(const CrossCtx& c, const int (&ib)[3]
 
 // General path for one particle that left its cell (or whose cell lies
 // outside the box): boundary rules, zigzag with relay point, charge at the
-// stored cell; the final record is written here.  CURV = false: no
+// stored cell; the final record is written here.  A particle that ends in no
+// cell of the grid is reported and dropped.  CURV = false: no
 // cylinder or sphere to test.  JD = false: charge only (no zigzag current).
 template <int B, bool DEP = true, bool CURV = true, bool JD = true>
 __device__ __forceinline__ int cross_one(const Geo& g, unsigned long long* box, const int (&o)[3], const Sink& sk,
@@ -757,7 +758,15 @@ __device__ __forceinline__ int cross_one(const Geo& g, unsigned long long* box, 
   // slab (its stored position, the slab's periodic wrap, is its position
   // there); its current stays here, in the guard planes that the ranks
   // exchange and fold, and its charge is deposited by the receiver
-  const bool migrant = c.ob != nullptr && az.crossed && !escaped && !absorbed;
+  // the boundary rules wrap or reflect once: a displacement longer than the
+  // axis ends in no cell of the grid, and packed it would be another
+  // particle's cell or an index past every per-cell table
+  const bool lost = !escaped && !absorbed && ((unsigned)ax.nc >= (unsigned)g.nx || (unsigned)ay.nc >= (unsigned)g.ny ||
+                                              (unsigned)az.nc >= (unsigned)g.nz);
+  if (lost)
+    report_bad(c.status, sk.diag, SITE_FX_PUSH, c.slot_base + loc,
+               ax.nc + 100000LL * ay.nc + 10000000000LL * az.nc);
+  const bool migrant = c.ob != nullptr && az.crossed && !escaped && !absorbed && !lost;
   if (migrant) {
     const int dir = az.ac < 0 ? 0 : 1;
     const unsigned long long q = atomicAdd(&c.ob->count[2 * c.is + dir], 1ull);
@@ -774,7 +783,7 @@ __device__ __forceinline__ int cross_one(const Geo& g, unsigned long long* box, 
       atomicOr(c.status, ST_OVERFLOW);
     }
   }
-  const bool dead = escaped || absorbed || migrant;
+  const bool dead = escaped || absorbed || migrant || lost;
   const uint32_t nc = dead ? DEAD : pack(g, ax.nc, ay.nc, az.nc);
   c.gpos[loc] = make_float4(ax.nf, ay.nf, az.nf, __int_as_float((int)nc));
   c.gvx[loc] = vx;

@@ -75,6 +75,10 @@ __device__ __forceinline__ int lcs_axis(const LcsGeo& G, int d, int tile, int i)
   return (l >= 0 && l < G.bc[d]) ? l : -1;
 }
 
+__device__ __forceinline__ bool lcs_in_grid(const LcsGeo& G, int i, int j, int k) {
+  return (unsigned)i < (unsigned)G.n[0] && (unsigned)j < (unsigned)G.n[1] && (unsigned)k < (unsigned)G.n[2];
+}
+
 // Box cell of cell (i,j,k) in the sort box of tile (tx,ty,tz), or -1.
 __device__ __forceinline__ int lcs_box_cell(const LcsGeo& G, int tx, int ty, int tz, int i, int j, int k) {
   int a = lcs_axis(G, 0, tx, i), b = lcs_axis(G, 1, ty, j), c = lcs_axis(G, 2, tz, k);
@@ -119,7 +123,8 @@ __global__ void __launch_bounds__(PUSH_THREADS, 2) k_lcs_count(const float4* __r
                                                             const int64_t* __restrict__ tp, Geo g, LcsGeo G,
                                                             uint32_t* __restrict__ wcnt, uint32_t* __restrict__ cnt,
                                                             int* stray, int* nstray,
-                                                            unsigned long long* __restrict__ slist) {
+                                                            unsigned long long* __restrict__ slist, int* status,
+                                                            long long* diag) {
   extern __shared__ uint32_t hist[];  // [PUSH_WARPS][nbc]
   const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5;
   for (int e = tid; e < PUSH_WARPS * G.nbc; e += PUSH_THREADS) hist[e] = 0;
@@ -148,6 +153,12 @@ __global__ void __launch_bounds__(PUSH_THREADS, 2) k_lcs_count(const float4* __r
       int i, j, k;
       unpack(g, cell, i, j, k);
       if (lcs_box_cell(G, tx, ty, tz, i, j, k) >= 0) continue;
+      // the key indexes per-cell tables: no key for a cell off the grid (the
+      // push leaves none)
+      if (!lcs_in_grid(G, i, j, k)) {
+        report_bad(status, diag, SITE_FX_SORT, tp[t] + r * PUSH_THREADS + tid, (long long)cell);
+        continue;
+      }
       const int q = atomicAdd(nstray, 1);
       if (q < STRAY_MAX)
         slist[q] = ((unsigned long long)cell_key(g, i, j, k) << 32) | (uint32_t)(tp[t] + r * PUSH_THREADS + tid);
@@ -490,7 +501,7 @@ __global__ void __launch_bounds__(PUSH_THREADS, 2) k_lcs_rank(const float4* __re
     if (cell == DEAD) continue;
     int i, j, k;
     unpack(g, cell, i, j, k);
-    if (lcs_box_cell(G, tx, ty, tz, i, j, k) >= 0) continue;
+    if (lcs_box_cell(G, tx, ty, tz, i, j, k) >= 0 || !lcs_in_grid(G, i, j, k)) continue;
     const unsigned long long first = (unsigned long long)cell_key(g, i, j, k) << 32;
     const uint32_t key = (uint32_t)(first >> 32);
     const int64_t td = key / (uint32_t)G.tcells;

@@ -3,7 +3,7 @@ a cell, many, and more than it takes (then the radix sort outside a graph)."""
 import numpy as np
 import pytest
 
-from ctca_b200.emses import Emses
+from ctca_b200.emses import Emses, EmsesError
 
 from helpers import build, case, rel_l2
 
@@ -87,3 +87,34 @@ def test_sort_with_strays(gpu, n, ppc, vth, over):
         assert np.array_equal(pa.view(np.uint8), pb.view(np.uint8))
     for g in runs:
         g.close()
+
+
+# (grid, outer boundary, velocity): displacements of more than two axis lengths
+# (ustep 2), where one wrap or reflection does not lead back into the grid
+@pytest.mark.parametrize("n,npbnd,v", [
+    ((2, 16, 16), 0, 2.2),
+    ((20, 18, 13), 0, -40.0),       # partial tiles
+    ((16, 16, 16), 1, 33.0),
+    ((16, 16, 16), 0, 3e30),
+])
+@pytest.mark.parametrize("axis", range(3))
+@pytest.mark.parametrize("sort", [False, True])
+def test_displacement_past_the_grid_is_reported_and_dropped(gpu, n, npbnd, v, axis, sort):
+    c = case(n=np.roll(n, axis), ppc=(6, 5), npbnd=(npbnd,) * 3, nfbnd=(npbnd,) * 3, e=False, b0=(0.0, 0.0, 0.0),
+             tile=(8, 8, 8))
+    cfg, eb, p, tp = build(c, 1.2)
+    p = p.copy()
+    m = int(tp[0]) // 2
+    p["v" + "xyz"[axis]][m] = v
+    with Emses(cfg) as g:
+        g.upload_particles(p, tp)
+        g.upload_field("eb", eb)
+        g.fx_load()
+        g.fx_step(2, sort)
+        with pytest.raises(EmsesError, match="outside the field arrays"):
+            g.synchronize()
+        # the others go on without it
+        g.fx_sort()
+        g.fx_step(2, True)
+        g.synchronize()
+        assert np.array_equal(g.fx_counts(), tp[:cfg.nspec] - np.array([1, 0]))
