@@ -233,7 +233,8 @@ struct Axis {
   bool dead, flip, crossed;
 };
 
-// The outer boundary rules for an "after" cell ac outside 0..n-1.
+// The outer boundary rules for an "after" cell ac outside 0..n-1.  They
+// wrap or reflect once: a displacement longer than the axis can leave nc outside 0..n-1.
 __device__ __forceinline__ Axis axis_boundary(int ib, float ob, int ac, float af, int n, int npbnd) {
   Axis o;
   o.dead = false;
@@ -387,13 +388,12 @@ __device__ __forceinline__ void put_j_global(Sink s, int i, int j, int k, V12 v,
 __device__ __forceinline__ void put_r_global(Sink s, int i, int j, int k, V8 v, float qfix) {
   for (int r = 0; r < NR; r++) {
     const long long f = to_fix(v.v[r], qfix);
-    if (f == 0) continue;
     const int ii = i + rdi(r), jj = j + rdj(r), kk = k + rdk(r);
     if (ii < -1 || jj < -1 || kk < -1 || ii > s.nx + 1 || jj > s.ny + 1 || kk > s.nz + 1) {
       report_bad(s.status, s.diag, SITE_FX_DEPOSIT, -1, ii + 100000LL * jj + 10000000000LL * kk);
       continue;
     }
-    atomicAdd(&s.acc_rho[s.fr.at(0, ii, jj, kk)], (unsigned long long)f);
+    if (f != 0) atomicAdd(&s.acc_rho[s.fr.at(0, ii, jj, kk)], (unsigned long long)f);
   }
 }
 
@@ -758,15 +758,7 @@ __device__ __forceinline__ int cross_one(const Geo& g, unsigned long long* box, 
   // slab (its stored position, the slab's periodic wrap, is its position
   // there); its current stays here, in the guard planes that the ranks
   // exchange and fold, and its charge is deposited by the receiver
-  // the boundary rules wrap or reflect once: a displacement longer than the
-  // axis ends in no cell of the grid, and packed it would be another
-  // particle's cell or an index past every per-cell table
-  const bool lost = !escaped && !absorbed && ((unsigned)ax.nc >= (unsigned)g.nx || (unsigned)ay.nc >= (unsigned)g.ny ||
-                                              (unsigned)az.nc >= (unsigned)g.nz);
-  if (lost)
-    report_bad(c.status, sk.diag, SITE_FX_PUSH, c.slot_base + loc,
-               ax.nc + 100000LL * ay.nc + 10000000000LL * az.nc);
-  const bool migrant = c.ob != nullptr && az.crossed && !escaped && !absorbed && !lost;
+  const bool migrant = c.ob != nullptr && az.crossed && !escaped && !absorbed;
   if (migrant) {
     const int dir = az.ac < 0 ? 0 : 1;
     const unsigned long long q = atomicAdd(&c.ob->count[2 * c.is + dir], 1ull);
@@ -783,8 +775,13 @@ __device__ __forceinline__ int cross_one(const Geo& g, unsigned long long* box, 
       atomicOr(c.status, ST_OVERFLOW);
     }
   }
-  const bool dead = escaped || absorbed || migrant || lost;
-  const uint32_t nc = dead ? DEAD : pack(g, ax.nc, ay.nc, az.nc);
+  const bool dead = escaped || absorbed || migrant;
+  // After a displacement longer than an axis the stored cell may be none of
+  // the grid; packed it would be another particle's cell or an index past every
+  // per-cell table.  Such a particle is dropped.
+  const bool off =
+      (unsigned)ax.nc >= (unsigned)g.nx || (unsigned)ay.nc >= (unsigned)g.ny || (unsigned)az.nc >= (unsigned)g.nz;
+  const uint32_t nc = dead || off ? DEAD : pack(g, ax.nc, ay.nc, az.nc);
   c.gpos[loc] = make_float4(ax.nf, ay.nf, az.nf, __int_as_float((int)nc));
   c.gvx[loc] = vx;
   c.gvy[loc] = vy;
@@ -856,7 +853,14 @@ __device__ __forceinline__ int cross_one(const Geo& g, unsigned long long* box, 
     float R[NR];
     R[2] = XY * Z; R[1] = XZ - R[2]; R[3] = YZ - R[2]; R[0] = Z - XZ - R[3];
     R[6] = XY * Z2; R[5] = XZ2 - R[6]; R[7] = YZ2 - R[6]; R[4] = Z2 - XZ2 - R[7];
-    put_r<B>(box, o, sk, ax.nc, ay.nc, az.nc, R, c.qfix);
+    // The cell comes from the packed one (fewer registers than the axes'), so
+    // that of a particle dropped as off the grid unpacks to a z index of no
+    // array, and the bounds check of the global deposit reports it.  (A report
+    // of its own here or above cost the push 4 to 16 % where many particles
+    // cross; this way it is unchanged.)
+    int ci, cj, ck;
+    unpack(g, nc, ci, cj, ck);
+    put_r<B>(box, o, sk, ci, cj, ck, R, c.qfix);
   }
   return escaped ? 1 : 0;
 }
