@@ -103,9 +103,8 @@ __device__ __forceinline__ bool split_coord(double x, int n, int& c, float& o) {
   double f = floor(x);
   c = (int)f;
   o = (float)(x - f);
-  const float below_one = 0.99999994f;
-  if (o >= 1.0f) o = below_one;
-  if (c == n && x == (double)n) { c = n - 1; o = below_one; }
+  if (o >= 1.0f) o = BELOW_ONE;
+  if (c == n && x == (double)n) { c = n - 1; o = BELOW_ONE; }
   return c >= 0 && c < n;
 }
 

@@ -233,8 +233,12 @@ struct Axis {
   bool dead, flip, crossed;
 };
 
-// The outer boundary rules for an "after" cell ac outside 0..n-1.  They
-// wrap or reflect once: a displacement longer than the axis can leave nc outside 0..n-1.
+constexpr float BELOW_ONE = 0.99999994f;  // the largest offset
+
+// The outer boundary rules for an "after" cell ac outside 0..n-1.  A
+// reflection that ends exactly on the upper face, x = n, stays in the last
+// cell, as a record loaded there does.  The rules wrap or reflect once: a
+// displacement longer than the axis can leave nc outside 0..n-1.
 __device__ __forceinline__ Axis axis_boundary(int ib, float ob, int ac, float af, int n, int npbnd) {
   Axis o;
   o.dead = false;
@@ -248,6 +252,7 @@ __device__ __forceinline__ Axis axis_boundary(int ib, float ob, int ac, float af
       int rc_ = af > 0.f ? -ac - 1 : -ac;
       float rf_ = af > 0.f ? 1.0f - af : 0.0f;
       if (rf_ >= 1.0f) { rf_ = 0.f; rc_ += 1; }
+      if (rc_ == n && rf_ == 0.f) { rf_ = BELOW_ONE; rc_ -= 1; }
       o.ac = rc_; o.af = rf_; o.ia = 0; o.rc = 0; o.rf = 0.f;
       o.nc = rc_; o.nf = rf_; o.flip = true;
     } else {
@@ -262,6 +267,7 @@ __device__ __forceinline__ Axis axis_boundary(int ib, float ob, int ac, float af
       int rc_ = af > 0.f ? 2 * n - ac - 1 : 2 * n - ac;
       float rf_ = af > 0.f ? 1.0f - af : 0.0f;
       if (rf_ >= 1.0f) { rf_ = 0.f; rc_ += 1; }
+      if (rc_ == n && rf_ == 0.f) { rf_ = BELOW_ONE; rc_ -= 1; }
       o.ac = rc_; o.af = rf_; o.ia = n - 1; o.rc = n; o.rf = 0.f;
       o.nc = rc_; o.nf = rf_; o.flip = true;
     } else {

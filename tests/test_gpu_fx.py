@@ -223,6 +223,37 @@ def test_fx_em_step_vs_oracle(gpu):
     g.close()
 
 
+@pytest.mark.parametrize("axis", range(3))
+@pytest.mark.parametrize("sort", [False, True])
+def test_reflection_onto_the_face_stays_in_the_grid(gpu, axis, sort):
+    """A particle half a cell from a reflecting face with a displacement of
+    exactly half a cell ends on the face, x = n: it stays in the last cell and
+    comes back half a cell in the next step, as the oracle's does."""
+    c = case(n=(16, 12, 10), ppc=(6, 5), npbnd=(1, 1, 1), nfbnd=(1, 1, 1), e=False, b0=(0.0, 0.0, 0.0), tile=(8, 8, 8))
+    cfg, eb, p, tp = build(c)
+    p = p.copy()
+    n = c.n[axis]
+    for d in range(3):
+        p["xyz"[d]][0], p["v" + "xyz"[d]][0] = (n - 0.5, 0.25) if d == axis else (4.5, 0.0)
+    with Emses(cfg) as g:
+        g.upload_particles(p, tp)
+        g.upload_field("eb", eb)
+        g.fx_load()
+        g.fx_store()
+        o = O.Oracle(cfg, *g.download_particles(), eb)
+        g.fx_load()
+        for x in (n, n - 0.5):
+            g.fx_step(2, sort)
+            oracle_step(o)
+            g.fx_store()
+            q, tq = g.download_particles()
+            assert np.array_equal(tq, tp)
+            mine = q[(np.abs(q["v" + "xyz"[axis]]) == 0.25)]
+            assert mine.size == 1 and abs(mine["xyz"[axis]][0] - x) < 1e-6
+            assert rel_l2(g.download_field("rho"), o.f["rho"]) < RHOJ_TOL
+            assert rel_l2(g.download_field("aj"), o.f["aj"]) < RHOJ_TOL
+
+
 def test_fx_empty_species_tracks_oracle(gpu):
     """A species without particles: steps and sorts (tile-local) leave it
     empty and the other species tracks the oracle."""
