@@ -97,6 +97,9 @@ struct FxState {
   float* vz2 = nullptr;
   int64_t* count_d = nullptr;       // device live-particle counts per species (last sort)
   int64_t* slots_d = nullptr;       // device slot counts per species (padded regions)
+  int64_t* counts_mem = nullptr;    // their allocation
+  int64_t* count2_d = nullptr;      // both of the layout a tile sort is making (swapped in once it is through)
+  int64_t* slots2_d = nullptr;
   int64_t* tile_start = nullptr;    // [nspec][ntiles+1] sorted ranks of each tile's first particle
   int64_t* tile_pad = nullptr;      // [nspec][ntiles+1] first slot of each tile's padded region
   int64_t* chunk_start = nullptr;   // [nspec][ntiles+1] first push CTA of each tile

@@ -486,8 +486,12 @@ int fx_alloc(emsesg_ctx* ctx) {
   EMSESG_CUDA(ctx, cudaMalloc(&f.vx2, cap * sizeof(float)));
   EMSESG_CUDA(ctx, cudaMalloc(&f.vy2, cap * sizeof(float)));
   EMSESG_CUDA(ctx, cudaMalloc(&f.vz2, cap * sizeof(float)));
-  EMSESG_CUDA(ctx, cudaMalloc(&f.count_d, EMSESG_ISPEC * sizeof(int64_t)));
-  EMSESG_CUDA(ctx, cudaMalloc(&f.slots_d, EMSESG_ISPEC * sizeof(int64_t)));
+  EMSESG_CUDA(ctx, cudaMalloc(&f.counts_mem, 4 * EMSESG_ISPEC * sizeof(int64_t)));
+  EMSESG_CUDA(ctx, cudaMemsetAsync(f.counts_mem, 0, 4 * EMSESG_ISPEC * sizeof(int64_t), ctx->stream));
+  f.count_d = f.counts_mem;
+  f.slots_d = f.counts_mem + EMSESG_ISPEC;
+  f.count2_d = f.counts_mem + 2 * EMSESG_ISPEC;
+  f.slots2_d = f.counts_mem + 3 * EMSESG_ISPEC;
   EMSESG_CUDA(ctx, cudaMalloc(&f.tile_start, (int64_t)c.nspec * (f.ntiles + 1) * sizeof(int64_t)));
   EMSESG_CUDA(ctx, cudaMalloc(&f.tile_pad, (int64_t)c.nspec * (f.ntiles + 1) * sizeof(int64_t)));
   EMSESG_CUDA(ctx, cudaMalloc(&f.chunk_start, (int64_t)c.nspec * (f.ntiles + 1) * sizeof(int64_t)));
@@ -559,7 +563,7 @@ void fx_free(emsesg_ctx* ctx) {
   FxState& f = ctx->fx;
   cudaFree(f.pos); cudaFree(f.vx); cudaFree(f.vy); cudaFree(f.vz);
   cudaFree(f.pos2); cudaFree(f.vx2); cudaFree(f.vy2); cudaFree(f.vz2);
-  cudaFree(f.count_d); cudaFree(f.slots_d); cudaFree(f.tile_start); cudaFree(f.tile_pad); cudaFree(f.accum_mem);
+  cudaFree(f.counts_mem); cudaFree(f.tile_start); cudaFree(f.tile_pad); cudaFree(f.accum_mem);
   cudaFree(f.chunk_start); cudaFree(f.chunks); cudaFree(f.defer);
   cudaFree(f.fnode); cudaFree(f.fnode2);
   cudaFree(f.diag);
@@ -588,9 +592,11 @@ int64_t sort_slots(emsesg_ctx* ctx, int is) {
 }
 }  // namespace
 
-// The tile-local counting sort (fx_sort.cuh).  Sets *done = false, having
-// changed nothing, when a particle left its tile's sort box; the caller then
-// sorts with the radix path.
+// The tile-local counting sort (fx_sort.cuh).  Sets *done = false when more
+// particles of a species than STRAY_MAX left their tiles' sort boxes; the
+// caller then sorts with the radix path.  By then species before that one are
+// sorted into the second buffers, with their counts in count2_d and slots2_d:
+// the layout in use and its counts are as they were.
 int fx_local_sort(emsesg_ctx* ctx, bool* done) {
   *done = false;
   FxState& f = ctx->fx;
@@ -636,8 +642,8 @@ int fx_local_sort(emsesg_ctx* ctx, bool* done) {
       EMSESG_CUDA(ctx, cudaMemsetAsync(ts2, 0, T1 * sizeof(int64_t), ctx->stream));
       EMSESG_CUDA(ctx, cudaMemsetAsync(tp2, 0, T1 * sizeof(int64_t), ctx->stream));
       EMSESG_CUDA(ctx, cudaMemsetAsync(f.chunk_start + is * T1, 0, T1 * sizeof(int64_t), ctx->stream));
-      EMSESG_CUDA(ctx, cudaMemsetAsync(f.count_d + is, 0, sizeof(int64_t), ctx->stream));
-      EMSESG_CUDA(ctx, cudaMemsetAsync(f.slots_d + is, 0, sizeof(int64_t), ctx->stream));
+      EMSESG_CUDA(ctx, cudaMemsetAsync(f.count2_d + is, 0, sizeof(int64_t), ctx->stream));
+      EMSESG_CUDA(ctx, cudaMemsetAsync(f.slots2_d + is, 0, sizeof(int64_t), ctx->stream));
       continue;
     }
     const int64_t off = f.base[is];
@@ -676,8 +682,8 @@ int fx_local_sort(emsesg_ctx* ctx, bool* done) {
                     f.lcs_celltot, (unsigned long long*)f.lcs_tiletot, stray);
     EMSESG_LAUNCH(ctx, "lcs_tiles", k_lcs_tiles, 1, 1024, STRAY_MAX * sizeof(unsigned long long), f.lcs_tiletot,
                   f.lcs_celltot, f.ntiles, ts2, tp2, f.chunk_start + is * T1,
-                  (int4*)f.chunks + is * f.nchunk_max, f.chunk_rows, f.count_d + is,
-                  f.slots_d + is, stray, nstray, f.lcs_slist, (int)tcells);
+                  (int4*)f.chunks + is * f.nchunk_max, f.chunk_rows, f.count2_d + is,
+                  f.slots2_d + is, stray, nstray, f.lcs_slist, (int)tcells);
     EMSESG_LAUNCH(ctx, "lcs_bases", k_lcs_bases, (unsigned)f.ntiles, CELL_THREADS, 0, cnt, f.lcs_celltot, g, G[is],
                   ts2, tp2, bas, f.lcs_inv + off, stray, nstray, f.lcs_regend);
     EMSESG_LAUNCH(ctx, "lcs_rank", k_lcs_rank, (unsigned)f.ntiles, PUSH_THREADS, lsm, f.pos + off,
@@ -709,7 +715,7 @@ int fx_local_sort(emsesg_ctx* ctx, bool* done) {
     if (f.capture)
       EMSESG_LAUNCH(ctx, "lcs_keep", k_lcs_keep, 4 * 148, 256, 0, stray, f.pos + off, f.vx + off, f.vy + off,
                     f.vz + off, f.tile_start + is * T1, f.tile_pad + is * T1, f.ntiles, f.pos2 + off, f.vx2 + off,
-                    f.vy2 + off, f.vz2 + off, ts2, tp2, f.lcs_inv + off);
+                    f.vy2 + off, f.vz2 + off, ts2, tp2, f.lcs_inv + off, f.count2_d + is, f.slots2_d + is);
   }
   std::swap(f.pos, f.pos2);
   std::swap(f.vx, f.vx2);
@@ -717,6 +723,8 @@ int fx_local_sort(emsesg_ctx* ctx, bool* done) {
   std::swap(f.vz, f.vz2);
   std::swap(f.tile_start, f.tile_start2);
   std::swap(f.tile_pad, f.tile_pad2);
+  std::swap(f.count_d, f.count2_d);
+  std::swap(f.slots_d, f.slots2_d);
   for (int is = 0; is < c.nspec; is++) f.ntail[is] = 0;  // merged into the regions
   f.chunks_stale = false;
   *done = true;

@@ -747,23 +747,27 @@ __global__ void __launch_bounds__(Cfg::T, Cfg::CTAS) k_lcs_move(const float4* __
   move_tile<Cfg, 32>(pos, vx, vy, vz, inv, pos2, vx2, vy2, vz2, Ld, Ls, tp[t], tp2[t], ns > 0, msm, wlo);
 }
 
-// Inside a CUDA graph the host cannot switch to the radix sort when more
-// than STRAY_MAX particles of a species have left their sort boxes; the sort
-// kernels above then return
-// at once and this one keeps the current order instead: the new buffers get
-// the old regions slot for slot (inv = identity).  The push handles a
-// particle outside its tile's box on its general path (global gather and
-// deposits), so the step stays correct, only slower, until the next sort
-// outside a graph.  Does nothing when the sort went through.
+// Inside a CUDA graph the host cannot switch to the radix sort when more than
+// STRAY_MAX particles of a species have left their sort boxes; the sort
+// kernels above then return at once and this one keeps the current order
+// instead: the new buffers get the old regions slot for slot (inv = identity)
+// and their counts.  The push handles a particle outside its tile's box on its
+// general path (global gather and deposits), so the step stays correct, only
+// slower, until the next sort outside a graph.  Does nothing when the sort
+// went through.
 __global__ void __launch_bounds__(256) k_lcs_keep(const int* stray, const float4* __restrict__ pos,
                                                   const float* __restrict__ vx, const float* __restrict__ vy,
                                                   const float* __restrict__ vz, const int64_t* __restrict__ ts,
                                                   const int64_t* __restrict__ tp, int64_t ntiles, float4* pos2,
                                                   float* vx2, float* vy2, float* vz2, int64_t* ts2, int64_t* tp2,
-                                                  uint32_t* inv) {
+                                                  uint32_t* inv, int64_t* count2, int64_t* slots2) {
   if (!*stray) return;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i0 == 0) {
+    *count2 = ts[ntiles];
+    *slots2 = tp[ntiles];
+  }
   for (int64_t t = i0; t <= ntiles; t += stride) {
     ts2[t] = ts[t];
     tp2[t] = tp[t];

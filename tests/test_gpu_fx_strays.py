@@ -3,7 +3,7 @@ a cell, many, and more than it takes (then the radix sort outside a graph)."""
 import numpy as np
 import pytest
 
-from ctca_b200.emses import Emses, EmsesError
+from ctca_b200.emses import FX_ROW_SLOTS, Emses, EmsesError
 
 from helpers import build, case, rel_l2
 
@@ -87,6 +87,44 @@ def test_sort_with_strays(gpu, n, ppc, vth, over):
         assert np.array_equal(pa.view(np.uint8), pb.view(np.uint8))
     for g in runs:
         g.close()
+
+
+def test_fallback_on_a_later_species_keeps_the_first(gpu):
+    """Too many strays of the second species: the first, already through the
+    tile sort, goes to the radix sort too, from its old layout.  Its tiles
+    hold a few particles more than 9 rows at the load (13 ppc) and some of
+    them fewer after the steps, so the new layout has fewer slots than the old
+    one has in use."""
+    tile = (8, 8, 8)
+    c = case(n=(32, 32, 32), ppc=(13, 1), vth_scale=3.0, tile=tile)
+    cfg, eb, p, tp = build(c, 1.2)
+    p = p.copy()
+    for f in ("vx", "vy", "vz"):
+        p[f][tp[0]:] *= 600.0
+    with Emses(cfg) as g:
+        g.upload_particles(p, tp)
+        g.upload_field("eb", eb)
+        g.fx_load()
+        g.fx_store()
+        p0, _ = g.download_particles()
+        for _ in range(4):
+            g.fx_step(2, False)
+        g.fx_store()
+        p1, t1 = g.download_particles()
+        n0 = int(t1[0])
+        assert strays(cfg, tile, p0[:n0], p1[:n0]) <= STRAY_MAX < strays(cfg, tile, p0[n0:], p1[n0:])
+        rows = [int(np.sum(-(-np.bincount(key_of(cfg, tile, q[:n0]) // 512) // FX_ROW_SLOTS))) for q in (p0, p1)]
+        assert rows[1] < rows[0]
+        g.fx_sort()
+        assert np.array_equal(g.fx_counts(), t1)
+        g.fx_store()
+        p2, t2 = g.download_particles()
+    assert np.array_equal(t1, t2)
+    for u, v in ((p1[:n0], p2[:n0]), (p1[n0:], p2[n0:])):
+        assert np.all(np.diff(key_of(cfg, tile, v)) >= 0)
+        ku, kv = (np.lexsort([q[f] for f in FIELDS]) for q in (u, v))
+        for f in FIELDS:
+            assert np.array_equal(u[f][ku], v[f][kv])
 
 
 # (grid, outer boundary, velocity): displacements of more than two axis lengths
