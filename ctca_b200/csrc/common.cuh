@@ -204,6 +204,7 @@ struct emsesg_ctx {
   emsesg_config cfg;
   emsesg_config* d_cfg = nullptr;      // device copy of cfg for the kernels
   int device = 0;
+  int sms = 148;                       // multiprocessors of the device
   cudaStream_t stream = nullptr;
   // host transfers beside the step (emsesg_fx_step_download,
   // emsesg_upload_field_async): a side stream, the event after a step's

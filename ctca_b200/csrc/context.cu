@@ -130,6 +130,7 @@ extern "C" int emsesg_create(const emsesg_config* cfg, emsesg_ctx** out) {
   int rc = validate_config(ctx, cfg);
   if (rc) { delete ctx; return rc; }
   cudaError_t e = cudaGetDevice(&ctx->device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     rc = check_cuda(ctx, e, "stream");

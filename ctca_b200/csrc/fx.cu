@@ -703,12 +703,14 @@ int fx_local_sort(emsesg_ctx* ctx, bool* done) {
                     f.lcs_inv + off, f.pos2 + off, f.vx2 + off, f.vy2 + off, f.vz2 + off, stray);
       return (int)EMSESG_OK;
     };
-    const int64_t mean = ctx->totalp[is] + nt, per_row = PUSH_THREADS * f.ntiles;
+    const int64_t most = ctx->totalp[is] + nt, per_row = PUSH_THREADS * f.ntiles;
+    const double full = (double)most * tcells / ((double)c.nx * c.ny * c.nz * PUSH_THREADS);  // rows of a full tile
+    auto waves = [&](auto cfg) { return f.ntiles / ((int64_t)decltype(cfg)::CTAS * ctx->sms); };
     int mrc;
-    if (mean <= MOVE_SMALL_ROWS * per_row)
-      mrc = f.ntiles >= MOVE_SMALL_TILES ? move(MoveSmallMany()) : move(MoveSmall());
-    else if (mean <= MOVE_MID_ROWS * per_row)
-      mrc = f.ntiles >= MOVE_MID_TILES ? move(MoveMidMany()) : move(MoveMid());
+    if (most <= MOVE_SMALL_ROWS * per_row)
+      mrc = waves(MoveSmallMany()) >= MOVE_SMALL_WAVES ? move(MoveSmallMany()) : move(MoveSmall());
+    else if (most <= MOVE_MID_ROWS * per_row)
+      mrc = waves(MoveMidMany()) >= MOVE_MID_WAVES && full <= MOVE_MID_MANY_ROWS ? move(MoveMidMany()) : move(MoveMid());
     else
       mrc = move(MoveBig());
     if (mrc) return mrc;

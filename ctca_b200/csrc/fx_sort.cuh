@@ -549,19 +549,29 @@ struct MoveCfg {
 using MoveBig = MoveCfg<3200, 2560, false, 2, PUSH_THREADS, 1>;      // up to 80 rows of 40 columns
 using MoveMid = MoveCfg<2240, 1792, false, 3, PUSH_THREADS, 1>;   // up to 56 rows of 40 columns, two groups in flight
 using MoveSmall = MoveCfg<1600, 1280, true, 2, PUSH_THREADS, 1>;     // up to 40 rows of 40 columns
-// With many tiles, one buffer and three CTAs of fewer threads a multiprocessor:
-// the other CTAs' copies and writes fill the waits, and no barrier holds 23
-// warps.  Small, per species: 75x42x61 x 40/20 ppc (480 tiles) 177 -> 136 us,
-// 80x64x96 x 32 ppc (960) 343 -> 286; with 64 tiles (32^3 x 16 ppc) the fewer
-// threads of a tile show, 39 -> 50, so it starts where the tiles fill all the
-// CTAs once.  Mid: 128^3 x 64 ppc (4096 tiles) 2.32 -> 2.12 ms; 64^3 (512) 0.34
-// -> 0.39, so four times that.
+// With many tiles, one buffer and three CTAs of fewer threads a
+// multiprocessor: the other CTAs' copies and writes fill the waits, and no
+// barrier holds 23 warps.  us per sort, the shape above -> this one:
+//   Small (8-cell tiles of 3 / 14 / 30 rows): 125 tiles 46 -> 50, 54 -> 70,
+//     81 -> 107; 512 tiles 163 -> 104, 197 -> 167, 289 -> 273; 1728 tiles 490
+//     -> 228, 582 -> 371, 861 -> 651.  It starts where the tiles fill all the
+//     CTAs once.
+//   Mid (40 rows): 512 tiles 378 -> 388 (a second, nearly empty wave), 1000
+//     tiles 668 -> 626, 1728 1118 -> 940, 2197 1443 -> 1178, 4096 2627 -> 2208.
+//     It starts where such a wave costs less than it brings, at four full
+//     ones.
+//   Its windows hold 48 rows; a tile of more is gathered unstaged.  At 46 / 46.6
+//   / 47.3 / 48 rows a tile: 4096 tiles 3046 -> 2609, 3210 -> 2673, 3285 -> 2906,
+//   3357 -> 3592; 2197 tiles 1656 -> 1386, 1736 -> 1431, 1786 -> 1596, 1830 ->
+//   2049.  So up to 47 rows of a full tile at the mean density (the mean over
+//   the tiles is less where the grid's last tiles are partial).
 using MoveSmallMany = MoveCfg<1600, 1280, true, 1, 384, 3>;
 using MoveMidMany = MoveCfg<1920, 1536, false, 1, 256, 3>;  // up to 48 rows of 40 columns
 constexpr int MOVE_SMALL_ROWS = 32;              // mean rows per tile up to which MoveSmall is used
 constexpr int MOVE_MID_ROWS = 48;                // then MoveMid up to this mean
-constexpr int MOVE_SMALL_TILES = 3 * 148;        // tiles from which the ...Many shapes are used
-constexpr int MOVE_MID_TILES = 4 * 3 * 148;
+constexpr int MOVE_MID_MANY_ROWS = 47;           // rows of a full tile up to which MoveMidMany is used
+constexpr int MOVE_SMALL_WAVES = 1;              // waves of CTAs from which the ...Many shapes are used
+constexpr int MOVE_MID_WAVES = 4;
 constexpr int MOVE_MAXGROUPS = PUSH_THREADS / 32;
 template <class Cfg>
 inline int move_smem() { return Cfg::NBUF * Cfg::BUF; }
