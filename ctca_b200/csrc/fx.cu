@@ -2220,7 +2220,12 @@ int adj_reserve(emsesg_ctx* ctx, AdjWork& w, int nseg, int ckpt, int jsteps, int
   if ((int)w.inv.size() < ckpt) w.inv.resize((size_t)ckpt, nullptr);
   if (!w.lam) EMSESG_CUDA(ctx, cudaMalloc(&w.lam, 6 * cap * sizeof(float)));
   if (!w.lam2) EMSESG_CUDA(ctx, cudaMalloc(&w.lam2, 6 * cap * sizeof(float)));
-  if (!w.fwd) EMSESG_CUDA(ctx, cudaMalloc(&w.fwd, cap * sizeof(uint32_t)));
+  if (!w.fwd) {
+    // cleared once: a particle that the push dropped (off the grid) has no
+    // entry, and what it reads must be a slot (the call then ends in its error)
+    EMSESG_CUDA(ctx, cudaMalloc(&w.fwd, cap * sizeof(uint32_t)));
+    EMSESG_CUDA(ctx, cudaMemsetAsync(w.fwd, 0, cap * sizeof(uint32_t), ctx->stream));
+  }
   if (!w.gd) EMSESG_CUDA(ctx, cudaMalloc(&w.gd, 3 * nn * sizeof(float)));
   if (!w.gEd) EMSESG_CUDA(ctx, cudaMalloc(&w.gEd, 3 * nn * sizeof(double)));
   if (!w.gBd) EMSESG_CUDA(ctx, cudaMalloc(&w.gBd, 3 * nn * sizeof(double)));

@@ -15,7 +15,7 @@ the jump, not the derivative."""
 import numpy as np
 import pytest
 
-from ctca_b200.emses import Emses
+from ctca_b200.emses import Emses, EmsesError
 from oracle import oracle as O
 
 from helpers import build, case, rel_l2
@@ -174,3 +174,20 @@ def test_gpu_adjoint_on_the_16cube_copy_of_the_adjoint_workload(gpu):
     assert errs["loss"] < 1e-4
     for k in ("g0", "gE", "gB", "gv"):
         assert errs[k] < 1e-3, k
+
+
+@pytest.mark.parametrize("sort_every", [1, 4])
+def test_adjoint_of_a_run_that_loses_a_particle_is_refused(gpu, sort_every):
+    """A displacement past the grid: the forward pass drops the particle, the
+    reverse one, which meets it in the states before, stays in its arrays, and
+    the call returns the error."""
+    c = case(n=(16, 16, 16), ppc=(4, 4), seed=21, e=False, b0=(0.0, 0.0, 0.0), tile=(8, 8, 8))
+    cfg, eb, p, tp = build(c)
+    p = p.copy()
+    p["vx"][100] = 40.0
+    with Emses(cfg) as g:
+        g.upload_particles(p, tp)
+        g.upload_field("eb", eb)
+        g.fx_load()
+        with pytest.raises(EmsesError, match="outside the field arrays"):
+            g.fx_adjoint(4, 2, 2, sort_every, (4, 4, 4), (12, 12, 12), int(tp.sum()))
