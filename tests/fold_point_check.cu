@@ -44,8 +44,8 @@ int main() {
         for (auto& v : a) v = (long long)(rng() % 2000001) - 1000000;
         std::vector<double> d(a.begin(), a.end());
         for (auto& v : d) v *= 0.1;
-        // deposits lie within one node of the grid: the outer guards start at
-        // zero (the folds read only what the copies put there)
+        // every element starts random, the outer guards too, which a step
+        // leaves at zero
         std::vector<long long> sa = a;
         std::vector<double> sd = d;
         for (const SlabOp& o : ops) {
