@@ -435,23 +435,14 @@ __device__ __forceinline__ void put_r(unsigned long long* box, const int (&o)[3]
   }
 }
 
-template <bool SMEM>
-__device__ __forceinline__ void gather8(const float4* f0, const void* f1v, int64_t n5, int64_t sy, int64_t sz,
+// E and B from the global node field, corner weights times values.
+__device__ __forceinline__ void gather8(const float4* f0, const float4* f1, int64_t n5, int64_t sy, int64_t sz,
                                         const float (&w)[8], float (&e)[3], float (&b)[3]) {
   const int64_t idx[8] = {n5 + sz, n5 + sz + 1, n5 + sz + 1 + sy, n5 + sz + sy, n5, n5 + 1, n5 + 1 + sy, n5 + sy};
   float ex = 0.f, ey = 0.f, ez = 0.f, bx = 0.f, by = 0.f, bz = 0.f;
 #pragma unroll
   for (int c = 0; c < 8; c++) {
-    float4 p;
-    float2 q;
-    if (SMEM) {
-      p = f0[idx[c]];
-      q = reinterpret_cast<const float2*>(f1v)[idx[c]];
-    } else {
-      p = __ldg(&f0[idx[c]]);
-      float4 q4 = __ldg(&reinterpret_cast<const float4*>(f1v)[idx[c]]);
-      q = make_float2(q4.x, q4.y);
-    }
+    const float4 p = __ldg(&f0[idx[c]]), q = __ldg(&f1[idx[c]]);
     ex += p.x * w[c];
     ey += p.y * w[c];
     ez += p.z * w[c];
@@ -1350,7 +1341,7 @@ __global__ void k_fx_tail(FxPushArgs a, int is, int64_t tail0, int64_t ntail, in
   wv[6] = xy1 * z2; wv[5] = xz2 - wv[6]; wv[7] = yz2 - wv[6]; wv[4] = z2 - xz2 - wv[7];
   float fe[3], fb[3];
   const int64_t sy = g.nx + 1, sz = (int64_t)(g.nx + 1) * (g.ny + 1);
-  gather8<false>(a.f0, a.f1, ib + sy * jb + sz * kb, sy, sz, wv, fe, fb);
+  gather8(a.f0, a.f1, ib + sy * jb + sz * kb, sy, sz, wv, fe, fb);
   const float eex = fe[0] * qmp, eey = fe[1] * qmp, eez = fe[2] * qmp;
   const float bbx = fb[0] * qmp, bby = fb[1] * qmp, bbz = fb[2] * qmp;
   const float boris = 2.0f / (1.0f + bbx * bbx + bby * bby + bbz * bbz);
@@ -1377,11 +1368,9 @@ __global__ void k_fx_tail(FxPushArgs a, int is, int64_t tail0, int64_t ntail, in
 // is converted: what the row loop and the general path do for a particle
 // whose cell lies outside its tile's box -- the global gather and the kick,
 // then the general path with global deposits (a deposit takes the same
-// int64 value per node as through a tile's box).  The compiler may round
-// this kernel's kick otherwise than the row loop's (where it fuses a
-// multiply with an add), so such a particle can differ in the last bit from
-// the same step pushed in one launch.  One thread per 32-slot word of the
-// bitmap, which it clears.
+// int64 value per node as through a tile's box).  The same bits as from the
+// step pushed in one launch.  One thread per 32-slot word of the bitmap, which
+// it clears.
 template <int T, bool CURV, bool JD>
 __global__ void k_fx_deferred(FxPushArgs a, uint32_t* __restrict__ bits, int64_t nwords, int nspec) {
   constexpr int B = T + 2 * PG + 1;

@@ -1,4 +1,5 @@
-// slab.cuh -- device execution of the guard-fold slab operations (fold_ops.h).
+// slab.cuh -- device execution of the guard-fold slab operations (fold_ops.h),
+// one after the other (slab mode).
 #pragma once
 #include <algorithm>
 
@@ -43,13 +44,6 @@ __host__ __device__ __forceinline__ void slab_apply(T* __restrict__ a, const Sla
   }
 }
 
-template <typename T>
-__global__ void k_slab(T* __restrict__ a, SlabArgs s) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= s.count) return;
-  slab_apply(a, s, t);
-}
-
 // Up to SLAB_MULTI operations that touch no element another one of them
 // reads or writes, in one launch: the threads are dealt out to them in turn.
 constexpr int SLAB_MULTI = 4;
@@ -68,23 +62,6 @@ __global__ void k_slab_multi(SlabMulti<T> m) {
   int q = 0;
   while (q + 1 < m.n && t >= m.start[q + 1]) q++;
   slab_apply(m.a[q], m.s[q], t - m.start[q]);
-}
-
-template <typename T>
-int run_slab_ops(emsesg_ctx* ctx, T* a, const FieldDesc& f, const std::vector<SlabOp>& ops, const char* name) {
-  for (const SlabOp& o : ops) {
-    SlabArgs s;
-    s.o = o;
-    s.f = f;
-    int ax = o.axis, ea = ax == 0 ? 1 : 0, eb = ax == 2 ? 1 : 2;
-    int64_t na = o.hi[ea] - o.lo[ea] + 1, nb = o.hi[eb] - o.lo[eb] + 1;
-    s.count = (int64_t)o.depth * na * nb * o.nc;
-    if (s.count <= 0) continue;
-    int threads = 256;
-    int64_t blocks = (s.count + threads - 1) / threads;
-    EMSESG_LAUNCH(ctx, name, k_slab<T>, (unsigned)blocks, threads, 0, a, s);
-  }
-  return EMSESG_OK;
 }
 
 // Elements an operation writes and reads, as boxes of (component-blind)
