@@ -25,14 +25,14 @@
 // different cells, charge at the new cell).  So the divergent work of the few
 // runs with all lanes busy.
 //
-// What bounds it: issue slots (59 % of them) and shared-memory passes (65 %),
-// with the latency of 23 warps a SM between them; DRAM is at 35 %.  At 128^3 x
+// What bounds it: issue slots (60 % of them) and shared-memory passes (65 %),
+// with the latency of 23 warps a SM between them; DRAM is at 36 %.  At 128^3 x
 // 2 x 64 ppc a push took 7.45 ms with scalar FP32, out-of-place particles in
 // the run queue and rows by bulk copies on shared mbarriers (539 warp
 // instructions a row of 32); 6.81 ms with packed FP32 (f32x2), the
 // interpolation by lerps and the out-of-place list (455); 6.47 ms with rows
 // per warp, 32-bit slot indices and the field rows padded against bank
-// conflicts; 6.29 ms with the chunk table in place of a binary search (2.39
+// conflicts (433); 6.29 ms with the chunk table in place of a binary search (2.39
 // TB/s at 56 B a particle).  Not kept, at the same size: rows prefetched in
 // registers (spills, 6.61 ms), the lists out of line (12 ms: generic addresses
 // and an array argument in local memory), all lists at the end of the chunk
@@ -44,8 +44,8 @@
 // every conversion to fixed point is of one value; integer atomics commute.
 // Two runs on the same input give the same bits.
 
-// 23 warps, 6 on each SM sub-partition, at 80 registers a thread (a few values
-// spill on the general path): with 480-slot rows (16 warps, 128 registers) an
+// 23 warps, 6 on each SM sub-partition, at 80 registers a thread (408 bytes spill with the current, five local loads
+// and three stores a warp row, none without it): with 480-slot rows (16 warps, 128 registers) an
 // earlier form of the kernel took 8.16 ms, with 608 (20 warps, 96) 7.53, with
 // 736 7.20.
 constexpr int PUSH_THREADS = 736;           // pushing threads = slots per row
@@ -854,7 +854,7 @@ __device__ __forceinline__ int cross_one(const Geo& g, unsigned long long* box, 
     // that of a particle dropped as off the grid unpacks to a z index of no
     // array, and the bounds check of the global deposit reports it.  (A report
     // of its own here or above cost the push 4 to 16 % where many particles
-    // cross; this way it is unchanged.)
+    // cross; this way 0 %, and 1.2 % without the current.)
     int ci, cj, ck;
     unpack(g, nc, ci, cj, ck);
     put_r<B>(box, o, sk, ci, cj, ck, R, c.qfix);

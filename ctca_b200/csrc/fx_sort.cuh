@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(CELL_THREADS) k_lcs_celltot(const uint32_t* __
                                                               uint32_t* __restrict__ celltot,
                                                               int64_t* __restrict__ tiletot, const int* stray) {
   __shared__ uint32_t part[CELL_THREADS / 32];
-  if (*stray) return;  // a particle left its sort box: this sort is skipped (see fx_local_sort)
+  if (*stray) return;  // too many strays: this sort is skipped (see fx_local_sort)
   const int t = blockIdx.x, tid = threadIdx.x;
   int tx, ty, tz;
   tile_xyz(g, t, tx, ty, tz);

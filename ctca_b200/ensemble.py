@@ -16,7 +16,7 @@ region (rows per CTA: with fewer, a small grid's tiles spread over more
 SMs) of each grid-size class come from an autotuner that times the
 candidates on a batch of copies of the class's first run: tile and sort
 interval first, then the rows per CTA for the best of those (the CTA itself
-is fixed at 768 threads by the 736-slot rows of the layout).  Runs that do
+is fixed at 736 threads by the 736-slot rows of the layout).  Runs that do
 not fit in device memory together go in waves.
 
 Runs are drawn as stated for the ensemble workload: cubic periodic grids of

@@ -289,7 +289,9 @@ int emsesg_fx_load(emsesg_ctx* ctx);
 int emsesg_fx_store(emsesg_ctx* ctx);
 /* One step of the FP32 form: push of the tile regions and of the tail zone,
  * zigzag J and CIC rho into int64 fixed point, guard folds, FP64 rho / aj;
- * with do_sort, the re-sort after the push. */
+ * with do_sort, the re-sort after the push.  A particle that a displacement
+ * longer than an axis leaves in no cell of the grid is dropped, and the next
+ * emsesg_synchronize returns EMSESG_ERR_DEVICE. */
 int emsesg_fx_step(emsesg_ctx* ctx, int ustep, int do_sort);
 int emsesg_fx_sort(emsesg_ctx* ctx);
 /* emsesg_fx_step followed by the downloads of rho and aj (the arrays a field
@@ -303,11 +305,9 @@ int emsesg_fx_sort(emsesg_ctx* ctx);
  * so it overlaps with that step's sort.  With the FP32 form loaded the copy
  * goes in z chunks and the next FP32 step pushes its tile layers in parts,
  * each once its chunk is there; a particle outside its tile's box whose
- * node planes are not there yet is pushed after the last part, by a kernel
- * that may round its kick otherwise in the last bit (such a step agrees
- * with the step after a synchronous upload in counts, cells and liveness,
- * and up to those particles' last bits).  A synchronous emsesg_upload_field
- * of eb replaces a pending asynchronous one.  The two buffers change roles
+ * node planes are not there yet is pushed after the last part (such a step
+ * gives the bits of the step after a synchronous upload).  A synchronous
+ * emsesg_upload_field of eb replaces a pending asynchronous one.  The two buffers change roles
  * with every asynchronous upload: emsesg_fx_run takes a pending upload
  * before it captures or replays its graph and captures again when the eb
  * buffer changed; a batch (emsesg_batch_create) takes pending uploads before
